@@ -13,8 +13,12 @@
 //   dL/dR_{A,j} = sum_g sum_{mu on A} -2 v_rho d_j phi_mu G0_mu
 //                 - 2 sum_k v_k (d_j d_k phi_mu G0_mu + d_j phi_mu Gk_mu),
 //   with G0 = Phi D and Gk = (d_k Phi) D -- the forward contraction with a
-//   force epilogue (ctc_tiles.cuh), since d phi_mu / d R_A = -grad phi_mu for
-//   mu on atom A.
+//   force epilogue (ctc_fp64.cuh), since d phi_mu / d R_A = -grad phi_mu for
+//   mu on atom A.  Only the sum v_rho G0 + sum_k v_k Gk of the rows enters with
+//   d_j phi, and that is one row, w D with w = v_rho phi + v_grad . grad phi:
+//   two contraction rows per point (phi and w) instead of four, on tiles of 64
+//   points.  The AO kernel writes w, and dL/dD uses it too (W = 2 w - v_rho phi).
+#include "ctc_fp64.cuh"
 #include "ctc_tiles.cuh"
 
 namespace ctc {
@@ -66,10 +70,10 @@ __global__ void __launch_bounds__(kAdjScanThreads) adj_pair_offsets_kernel(TileB
 
 __global__ void __launch_bounds__(kAdjThreads)
     adjoint_dd_kernel(TileBatch tb, const int32_t* __restrict__ offsets, const double* __restrict__ v_rho,
-                      const double* __restrict__ v_grad, double* __restrict__ Cacc, int Mpad) {
+                      int wq, double* __restrict__ Cacc, int Mpad) {
   __shared__ double sA[2][kAdjK * kAdjLd];  // A of the row block, A of the column block
   __shared__ double sW[2][kAdjK * kAdjLd];  // W of the row block, W of the column block
-  __shared__ double sv[128][4];             // v_rho, 2 v_x, 2 v_y, 2 v_z per point
+  __shared__ double sv[128];                // v_rho per point
   const int TP = tb.TP;
   const int64_t ldq = (int64_t)TP * tb.Kcap;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -99,8 +103,7 @@ __global__ void __launch_bounds__(kAdjThreads)
       for (int j = tid; j < TP; j += kAdjThreads) {
         const int64_t oi = tb.out[(int64_t)t * TP + j];
         const bool ok = oi >= 0 && finite_point(tb.xyz + 3 * ((int64_t)t * TP + j));
-        sv[j][0] = ok ? v_rho[oi] : 0.0;
-        for (int d = 0; d < 3; ++d) sv[j][1 + d] = (ok && v_grad) ? 2.0 * v_grad[3 * oi + d] : 0.0;
+        sv[j] = ok ? v_rho[oi] : 0.0;
       }
       cur = t;
     }
@@ -119,9 +122,9 @@ __global__ void __launch_bounds__(kAdjThreads)
           const int kk = (side ? bj : bi) * kAdjB + k;
           const int64_t o = (int64_t)kk * TP + p0 + p;
           const double phi = ao[o];
-          const double* v = sv[p0 + p];
-          double w = v[0] * phi;
-          if (v_grad) w += v[1] * ao[ldq + o] + v[2] * ao[2 * ldq + o] + v[3] * ao[3 * ldq + o];
+          // W = v_rho phi + 2 v_grad . grad phi = 2 w - v_rho phi
+          const double vp = sv[p0 + p] * phi;
+          const double w = wq > 0 ? fma(2.0, ao[wq * ldq + o], -vp) : vp;
           sA[side][p * kAdjLd + k] = phi;
           sW[side][p * kAdjLd + k] = w;
         }
@@ -185,10 +188,11 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
   if (n > (int64_t)INT32_MAX) return fail(CTC_ERR_INVALID, "adjoint: at most 2^31-1 points per call");
   PointSrc src{};
   src.pts = d_points;
-  const int deriv = v_grad ? 2 : 1;
-  const int nq = v_grad ? 10 : 4;
-  const int nqa = (dLdR && v_grad) ? 4 : 1;
-  const int TP = 128 / nqa;
+  // AO quantities: what the outputs asked for need and no more
+  const int nq = v_grad ? (dLdR ? 11 : 2) : (dLdR ? 4 : 1);
+  const int deriv = dLdR ? 1 : 0;               // without v_grad
+  const int wq = v_grad ? (dLdR ? 10 : 1) : 0;  // quantity of w, 0: none
+  const int TP = dLdR && v_grad ? fp64_points(kFForce2) : fp64_points(kFForce1);
   const int Mpad = mol->Mpad;
   double* Cacc = nullptr;
   int rc;
@@ -199,17 +203,15 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
     Cacc = (double*)mol->ws_sl.p;
     CTC_CUDA_TRY(cudaMemsetAsync(Cacc, 0, cbytes, st));
   }
-  if (dLdR) {
-    rc = nqa == 4 ? ensure_smem_attr((const void*)fp64_tile_kernel<4, 1>, (int)kSmemFp64)
-                  : ensure_smem_attr((const void*)fp64_tile_kernel<1, 1>, (int)kSmemFp64);
-    if (rc != CTC_OK) return rc;
-  }
-  ForceArgs fa;
+  Fp64Args fa{};
   fa.v_rho = v_rho;
   fa.v_grad = v_grad;
   fa.ao_atom = mol->d_ao_atom;
   fa.dLdR = dLdR;
   fa.natom = mol->natom;
+  const std::function<int(const TileBatch&)> weighted = [&](const TileBatch& tb) {
+    return launch_ao_tiles_weighted(mol, tb, v_rho, v_grad, st);
+  };
   int nsm = 148;
   if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   rc = run_tiles(mol, src, n, TP, nq, deriv, st, [&](const TileBatch& tb) -> int {
@@ -219,22 +221,17 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
       int32_t* offsets = (int32_t*)mol->ws_adj.p;
       adj_pair_offsets_kernel<<<1, kAdjScanThreads, 0, st>>>(tb, offsets);
       CTC_CUDA_TRY(cudaGetLastError());
-      adjoint_dd_kernel<<<4 * nsm, kAdjThreads, 0, st>>>(tb, offsets, v_rho, v_grad, Cacc, Mpad);
+      adjoint_dd_kernel<<<4 * nsm, kAdjThreads, 0, st>>>(tb, offsets, v_rho, wq, Cacc, Mpad);
       CTC_CUDA_TRY(cudaGetLastError());
       mol->host_launches += 2;
     }
     if (dLdR) {
-      if (nqa == 4)
-        fp64_tile_kernel<4, 1><<<tb.C, kThreads, kSmemFp64, st>>>(tb, mol->d_D, Mpad, ctc_outputs{},
-                                                                 ctc_params{}, fa);
-      else
-        fp64_tile_kernel<1, 1><<<tb.C, kThreads, kSmemFp64, st>>>(tb, mol->d_D, Mpad, ctc_outputs{},
-                                                                 ctc_params{}, fa);
-      CTC_CUDA_TRY(cudaGetLastError());
+      const int r3 = v_grad ? launch_fp64<kFForce2>(mol, tb, fa, st) : launch_fp64<kFForce1>(mol, tb, fa, st);
+      if (r3 != CTC_OK) return r3;
       mol->host_launches += 1;
     }
     return CTC_OK;
-  });
+  }, v_grad ? &weighted : nullptr);
   if (rc != CTC_OK) return rc;
   if (dLdD) {
     const int64_t MM = (int64_t)mol->M * mol->M;

@@ -144,7 +144,7 @@ template <int DERIV, int TYPE, int TRACK>
 __device__ __forceinline__ void eval_typed(const DevSeg& sg, const double* __restrict__ alpha,
                                            const double* __restrict__ coef, double px, double py,
                                            double pz, double* __restrict__ o, int64_t ld_q,
-                                           int64_t ldc, int nq_out, unsigned* mx) {
+                                           int64_t ldc, int nq_out, unsigned* mx, const double* wv) {
   constexpr int L = TYPE == 0 ? 0 : (TYPE == 1 ? 1 : (TYPE <= 3 ? 2 : (TYPE <= 5 ? 3 : 4)));
   constexpr int NC = TYPE == 0 ? 1 : TYPE == 1 ? 3 : TYPE == 2 ? 6 : TYPE == 3 ? 5
                      : TYPE == 4 ? 10 : TYPE == 5 ? 7 : TYPE == 6 ? 15 : 9;
@@ -174,30 +174,30 @@ __device__ __forceinline__ void eval_typed(const DevSeg& sg, const double* __res
     Y[i] = Y[i - 1] * y;
     Z[i] = Z[i - 1] * z;
   }
-  if constexpr (TYPE == 0) ao_poly_0<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else if constexpr (TYPE == 1) ao_poly_1<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else if constexpr (TYPE == 2) ao_poly_2<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else if constexpr (TYPE == 3) ao_poly_3<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else if constexpr (TYPE == 4) ao_poly_4<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else if constexpr (TYPE == 5) ao_poly_5<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else if constexpr (TYPE == 6) ao_poly_6<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
-  else ao_poly_7<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx);
+  if constexpr (TYPE == 0) ao_poly_0<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else if constexpr (TYPE == 1) ao_poly_1<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else if constexpr (TYPE == 2) ao_poly_2<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else if constexpr (TYPE == 3) ao_poly_3<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else if constexpr (TYPE == 4) ao_poly_4<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else if constexpr (TYPE == 5) ao_poly_5<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else if constexpr (TYPE == 6) ao_poly_6<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
+  else ao_poly_7<DERIV, TRACK>(X, Y, Z, R0, R1, R2, o, ld_q, ldc, nq_out, mx, wv);
 }
 
 template <int DERIV, int TRACK>
 __device__ __forceinline__ void eval_dispatch(const DevSeg& sg, const double* __restrict__ alpha,
                                               const double* __restrict__ coef, double px, double py,
                                               double pz, double* __restrict__ o, int64_t ld_q,
-                                              int64_t ldc, int nq_out, unsigned* mx) {
+                                              int64_t ldc, int nq_out, unsigned* mx, const double* wv) {
   switch (sg.type) {
-    case 0: eval_typed<DERIV, 0, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    case 1: eval_typed<DERIV, 1, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    case 2: eval_typed<DERIV, 2, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    case 3: eval_typed<DERIV, 3, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    case 4: eval_typed<DERIV, 4, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    case 5: eval_typed<DERIV, 5, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    case 6: eval_typed<DERIV, 6, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
-    default: eval_typed<DERIV, 7, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx); break;
+    case 0: eval_typed<DERIV, 0, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    case 1: eval_typed<DERIV, 1, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    case 2: eval_typed<DERIV, 2, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    case 3: eval_typed<DERIV, 3, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    case 4: eval_typed<DERIV, 4, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    case 5: eval_typed<DERIV, 5, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    case 6: eval_typed<DERIV, 6, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
+    default: eval_typed<DERIV, 7, TRACK>(sg, alpha, coef, px, py, pz, o, ld_q, ldc, nq_out, mx, wv); break;
   }
 }
 
@@ -213,14 +213,22 @@ __device__ __forceinline__ void eval_dispatch(const DevSeg& sg, const double* __
 // or its points x phi (SLICE = 1, TP <= 256).  Every lane keeps the running
 // maximum of its values while it evaluates, so the exponents cost no second
 // pass over the block; slice_rows_kernel then writes the digit planes.
+//
+// SLICE = -1 or -2 is the adjoint's form: from the weights of the tile's points
+// (dL/drho, dL/dgrad rho at their original index) it also writes the row
+// w = v_rho phi + v_grad . grad phi, as quantity 10 behind the ten AO quantities
+// (-1) or as the only one besides phi (-2, dL/dD alone).  The contraction for
+// dL/dR then needs two rows per point instead of four, and dL/dD reads two
+// quantities instead of four.
 template <int DERIV, int SLICE>
 __global__ void __launch_bounds__(kAoThreads, 3)
     ao_tile_kernel(const DevSeg* __restrict__ segs, int nseg, const double* __restrict__ alpha,
                    const double* __restrict__ coef, TileBatch tb, int32_t* __restrict__ eexp,
-                   const int32_t* __restrict__ order) {
+                   const int32_t* __restrict__ order, const double* __restrict__ v_rho,
+                   const double* __restrict__ v_grad) {
   // per-warp maxima of the high word of |value| per row, [warp][row]
   constexpr int kMaxRows = 256;
-  __shared__ unsigned s_mx[SLICE ? kAoThreads / 32 : 1][SLICE ? kMaxRows : 1];
+  __shared__ unsigned s_mx[SLICE > 0 ? kAoThreads / 32 : 1][SLICE > 0 ? kMaxRows : 1];
   const int t = order ? order[blockIdx.x] : blockIdx.x;
   const int ns = tb.nsig[t], TP = tb.TP;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -233,16 +241,24 @@ __global__ void __launch_bounds__(kAoThreads, 3)
     const int j = pg + lane;
     const double px = xyz[3 * j], py = xyz[3 * j + 1], pz = xyz[3 * j + 2];
     unsigned mx[4] = {0u, 0u, 0u, 0u};
+    double wv[4] = {0.0, 0.0, 0.0, 0.0};
+    if (SLICE < 0) {
+      const int64_t oi = tb.out[(int64_t)t * TP + j];
+      if (oi >= 0) {
+        wv[0] = v_rho[oi];
+        for (int k = 0; k < 3; ++k) wv[1 + k] = v_grad[3 * oi + k];
+      }
+    }
     for (int i = warp; i < ns; i += kAoThreads / 32) {
       const DevSeg sg = segs[sl[i]];
       eval_dispatch<DERIV, SLICE>(sg, alpha, coef, px, py, pz, A + (int64_t)k0[i] * TP + j, ld_q, TP,
-                                  tb.nq, mx);
+                                  tb.nq, mx, wv);
     }
     if (SLICE == 4) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) s_mx[SLICE ? warp : 0][SLICE ? (pg / 32) * 128 + q * 32 + lane : 0] = mx[q];
+      for (int q = 0; q < 4; ++q) s_mx[SLICE > 0 ? warp : 0][SLICE > 0 ? (pg / 32) * 128 + q * 32 + lane : 0] = mx[q];
     } else if (SLICE == 1) {
-      s_mx[SLICE ? warp : 0][SLICE ? j : 0] = mx[0];
+      s_mx[SLICE > 0 ? warp : 0][SLICE > 0 ? j : 0] = mx[0];
     }
   }
   const int kt_true = tb.ktrue[t], kt = tb.kt[t];
@@ -251,13 +267,13 @@ __global__ void __launch_bounds__(kAoThreads, 3)
     const int q = idx / npad, r = idx % npad;
     A[q * ld_q + (int64_t)kt_true * TP + r] = 0.0;
   }
-  if (SLICE != 0) {
+  if (SLICE > 0) {
     __syncthreads();  // row maxima of every warp are in shared memory
     const int rows = split_tile_rows(TP, SLICE);
     for (int r = threadIdx.x; r < rows; r += kAoThreads) {
       unsigned m = 0u;
 #pragma unroll
-      for (int w = 0; w < kAoThreads / 32; ++w) m = max(m, s_mx[SLICE ? w : 0][SLICE ? r : 0]);
+      for (int w = 0; w < kAoThreads / 32; ++w) m = max(m, s_mx[SLICE > 0 ? w : 0][SLICE > 0 ? r : 0]);
       // |x| = 1.f 2^(E - 1023) < 2^(E - 1022) for the biased exponent E of the
       // largest |x| (frexp's exponent); a row of zeros gets 0
       const int E = (int)(m >> 20);
@@ -334,21 +350,27 @@ static int launch_ao_impl(const ctc_molecule* mol, const PointSrc& src, int64_t 
   return CTC_OK;
 }
 
-// Local-descriptor layout: out[(p * nq_out + q) * ld + ao]; AO columns beyond
-// M (padding up to Mpad) are left untouched and must be zeroed by the caller.
-int launch_ao(const ctc_molecule* mol, const PointSrc& src, int64_t n, int deriv, double* out,
-              int nq_out, int ld, cudaStream_t st) {
-  return launch_ao_impl(mol, src, n, deriv, out, nq_out, (int64_t)nq_out * ld, ld, st);
-}
-
 int launch_ao_tiles(const ctc_molecule* mol, const TileBatch& tb, int deriv, cudaStream_t st) {
   if (tb.C <= 0) return CTC_OK;
   const auto* sg = mol->d_segs;
+  const double *al = mol->d_alpha, *co = mol->d_coef;
   switch (deriv) {
-    case 0: ao_tile_kernel<0, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, mol->d_alpha, mol->d_coef, tb, nullptr, nullptr); break;
-    case 1: ao_tile_kernel<1, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, mol->d_alpha, mol->d_coef, tb, nullptr, nullptr); break;
-    default: ao_tile_kernel<2, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, mol->d_alpha, mol->d_coef, tb, nullptr, nullptr);
+    case 0: ao_tile_kernel<0, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
+    case 1: ao_tile_kernel<1, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
+    default: ao_tile_kernel<2, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr);
   }
+  CTC_CUDA_TRY(cudaGetLastError());
+  return CTC_OK;
+}
+
+int launch_ao_tiles_weighted(const ctc_molecule* mol, const TileBatch& tb, const double* v_rho,
+                             const double* v_grad, cudaStream_t st) {
+  if (tb.C <= 0) return CTC_OK;
+  const auto* sg = mol->d_segs;
+  const double *al = mol->d_alpha, *co = mol->d_coef;
+  if (tb.nq == 11) ao_tile_kernel<2, -1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, v_rho, v_grad);
+  else if (tb.nq == 2) ao_tile_kernel<1, -2><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, v_rho, v_grad);
+  else return fail(CTC_ERR_INVALID, "weighted AO tiles: unsupported quantity count");
   CTC_CUDA_TRY(cudaGetLastError());
   return CTC_OK;
 }
@@ -363,13 +385,13 @@ int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int der
   const auto* sg = mol->d_segs;
   const double *al = mol->d_alpha, *co = mol->d_coef;
   if (nqa == 4) {
-    if (deriv == 1) ao_tile_kernel<1, 4><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order);
-    else ao_tile_kernel<2, 4><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order);
+    if (deriv == 1) ao_tile_kernel<1, 4><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
+    else ao_tile_kernel<2, 4><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
   } else {
     switch (deriv) {
-      case 0: ao_tile_kernel<0, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order); break;
-      case 1: ao_tile_kernel<1, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order); break;
-      default: ao_tile_kernel<2, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order);
+      case 0: ao_tile_kernel<0, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr); break;
+      case 1: ao_tile_kernel<1, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr); break;
+      default: ao_tile_kernel<2, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
     }
   }
   CTC_CUDA_TRY(cudaGetLastError());

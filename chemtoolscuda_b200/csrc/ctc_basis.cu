@@ -51,6 +51,34 @@ __global__ void permute_density_kernel(const double* __restrict__ D, int M, int 
   out[e] = (i < M && j < M) ? D[(int64_t)perm[i] * M + perm[j]] : 0.0;
 }
 
+// *sym = 0 unless D is symmetric: |D_ij - D_ji| within 2^-50 of
+// (|D_ii| + |D_jj|) / 2, i.e. up to the rounding of a product C C^T whose two
+// halves were summed separately.  32 x 32 blocks on and above the diagonal.
+__global__ void __launch_bounds__(256) symmetry_kernel(const double* __restrict__ D, int Mpad, int32_t* sym) {
+  __shared__ double s_t[32][33];
+  const int bi = blockIdx.y * 32, bj = blockIdx.x * 32;
+  if (bj < bi) return;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int r = y; r < 32; r += 8) s_t[r][x] = D[(int64_t)(bj + r) * Mpad + bi + x];
+  __syncthreads();
+  const double dj = fabs(D[(int64_t)(bj + x) * Mpad + bj + x]);
+  bool ok = true;
+  for (int r = y; r < 32; r += 8) {
+    const double di = fabs(D[(int64_t)(bi + r) * Mpad + bi + r]);
+    // (a NaN in D compares false: the full sums then propagate it as they find it)
+    ok = ok && fabs(D[(int64_t)(bi + r) * Mpad + bj + x] - s_t[x][r]) <= 0x1p-51 * (di + dj);
+  }
+  if (!ok) *sym = 0;
+}
+
+int set_symmetry_flag(ctc_molecule* m, cudaStream_t st) {
+  CTC_CUDA_TRY(cudaMemsetAsync(m->d_sym, 1, sizeof(int32_t), st));  // any non-zero value
+  const unsigned nb = (unsigned)(m->Mpad / 32);
+  symmetry_kernel<<<dim3(nb, nb), 256, 0, st>>>(m->d_D, m->Mpad, m->d_sym);
+  CTC_CUDA_TRY(cudaGetLastError());
+  return CTC_OK;
+}
+
 int refresh_host_density(ctc_molecule* m) {
   if (!m->host_D_stale) return CTC_OK;
   const int M = m->M, Mp = m->Mpad;
@@ -154,16 +182,6 @@ void Scratch::release() {
   bytes = 0;
 }
 
-int64_t chunk_points(const ctc_molecule* mol, int nq_ao) {
-  // AO buffer (nq * Mpad doubles per point) plus int8 planes; keep a chunk
-  // around 2 GB so that the working set stays bounded for any basis size.
-  size_t per_pt = (size_t)mol->Mpad * (8 * (size_t)nq_ao + 16);
-  int64_t n = (int64_t)((size_t)2 << 30) / (int64_t)per_pt;
-  n = std::max<int64_t>(n, 128);
-  n = std::min<int64_t>(n, 1 << 20);
-  return (n / 128) * 128;
-}
-
 // The status word.  Kernels that can fail on the device (bounded waits of the
 // tensor-core pipeline) set the molecule's device word with atomicExch; it
 // stays set until it is reported.  After such kernels post_status enqueues a
@@ -176,6 +194,9 @@ static std::string status_message(int32_t code) {
            "the call's outputs are incomplete";
   if (code == 0x7201)
     return "a tile's significant functions exceeded the workspace capacity (status 0x7201); "
+           "the call's outputs are incomplete";
+  if (code == 0x7102)
+    return "a bounded wait of the FP64 contraction ran out (status 0x7102); "
            "the call's outputs are incomplete";
   return "kernel status " + std::to_string(code);
 }
@@ -434,7 +455,8 @@ int ctc_molecule_create(const ctc_basis* b, int32_t natom, const double* atom_xy
   ALLOC_COPY(m->d_ao_iperm, iperm.data(), iperm.size());
   ALLOC_COPY(m->d_ao_perm, m->ao_perm.data(), m->ao_perm.size());
 #undef ALLOC_COPY
-  if (cudaMalloc((void**)&m->d_status, sizeof(int32_t)) != cudaSuccess ||
+  if (cudaMalloc((void**)&m->d_sym, sizeof(int32_t)) != cudaSuccess || set_symmetry_flag(m, 0) != CTC_OK ||
+      cudaMalloc((void**)&m->d_status, sizeof(int32_t)) != cudaSuccess ||
       cudaMemset(m->d_status, 0, sizeof(int32_t)) != cudaSuccess ||
       cudaMallocHost((void**)&m->h_status, 4 * sizeof(int32_t)) != cudaSuccess ||
       cudaEventCreateWithFlags(&m->status_ev, cudaEventDisableTiming) != cudaSuccess ||
@@ -458,6 +480,7 @@ int ctc_molecule_destroy(ctc_molecule* m) {
   cudaFree(m->d_order);
   cudaFree(m->d_ao_atom);
   cudaFree(m->d_D);
+  cudaFree(m->d_sym);
   cudaFree(m->d_ao_iperm);
   cudaFree(m->d_ao_perm);
   cudaFree(m->d_Dsl);
@@ -493,6 +516,7 @@ int ctc_molecule_set_density_matrix(ctc_molecule* m, const double* d_D, void* st
   ctc::permute_density_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_D, M, Mp, m->d_ao_perm,
                                                                                m->d_D);
   CTC_CUDA_TRY(cudaGetLastError());
+  if (int rc = ctc::set_symmetry_flag(m, st); rc != CTC_OK) return rc;
   // the host copy (used only to build the ESP tables) is fetched again when needed
   m->host_D_stale = true;
   m->dsl_valid = false;

@@ -118,7 +118,7 @@ struct HostPipe {
 // tile's own K dimension (kt, padded to a multiple of 64).
 struct TileBatch {
   int C = 0;          // tiles in this chunk
-  int TP = 0;         // points per tile (32 or 128)
+  int TP = 0;         // points per tile (32, 64 or 128)
   int Kcap = 0;       // capacity of the compact K dimension (>= Mpad)
   int nq = 0;         // AO quantities per point (1, 4, 10)
   double* xyz = nullptr;    // [C][TP][3]
@@ -129,7 +129,9 @@ struct TileBatch {
   int32_t* segs = nullptr;  // [C][nseg] significant segment ids
   int32_t* k0 = nullptr;    // [C][nseg] compact offset of each significant segment
   int32_t* aomap = nullptr; // [C][Kcap] compact -> AO index, -1 for padding
-  double* ao = nullptr;     // [C][nq][TP][Kcap] AO values and derivatives
+  int32_t* order = nullptr; // [C] tiles, largest compact set first
+  int32_t* counter = nullptr; // zero when the contraction starts
+  double* ao = nullptr;     // [C][nq][Kcap][TP] AO values and derivatives
 };
 constexpr int kKtAlign = 64;
 
@@ -155,6 +157,7 @@ struct ctc_molecule {
   int32_t* d_order = nullptr;
   int32_t* d_ao_atom = nullptr;
   double* d_D = nullptr;                     // Mpad x Mpad, zero padded
+  int32_t* d_sym = nullptr;                  // 1: D is symmetric (set_symmetry_flag)
   // split-precision copy of D (4 int8 byte planes, row scales)
   int8_t* d_Dsl = nullptr;
   double* d_Dscale = nullptr;
@@ -191,15 +194,17 @@ namespace ctc {
 // ---- kernels / launchers (ctc_ao.cu) ----
 // AO block of every tile of a batch on its significant segments only.
 int launch_ao_tiles(const ctc_molecule* mol, const TileBatch& tb, int deriv, cudaStream_t st);
-// Same, and in the same kernel the int8 digit planes of the tile rows
+// The adjoint's form: nq = 11 (values, first and second derivatives and
+// w = v_rho phi + v_grad . grad phi as quantity 10) or nq = 2 (phi and w).
+int launch_ao_tiles_weighted(const ctc_molecule* mol, const TileBatch& tb, const double* v_rho,
+                             const double* v_grad, cudaStream_t st);
+// The plain form, and in the same kernel the int8 digit planes of the tile rows
 // (nqa = 4: 32 points x {phi, d phi}; nqa = 1: 128 points x phi) with one
 // exponent per row, for the tensor-core split path: planes [C][5][128][Kcap],
 // eexp [C][128].
 // order (optional) lists the tiles in the order the CTAs take them.
 int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int deriv, int nqa,
                            int8_t* planes, int32_t* eexp, const int32_t* order, cudaStream_t st);
-int launch_ao(const ctc_molecule* mol, const PointSrc& src, int64_t n, int deriv, double* out,
-              int nq_out, int ld, cudaStream_t st);
 // AO output in (nq, n, M) layout for ctc_eval_ao.
 int launch_ao_public(const ctc_molecule* mol, const PointSrc& src, int64_t n, int deriv,
                      double* out, cudaStream_t st);
@@ -216,20 +221,23 @@ int eval_local(ctc_molecule* mol, const PointSrc& src, int64_t n, int precision,
 
 // ---- tensor-core split path (ctc_tc.cu) ----
 int prepare_tc(ctc_molecule* mol, cudaStream_t st);
-// Workspace of the digit planes and row exponents of a chunk of tiles, and
-// the chunk's tile order (largest compact K first), computed here from tb.kt;
-// tc_local_tiles on the same batch uses all three.
+// Workspace of the digit planes and row exponents of a chunk of tiles;
+// tc_local_tiles on the same batch uses both.
 int tc_slice_workspace(ctc_molecule* mol, const TileBatch& tb, int nqa, cudaStream_t st,
-                       int8_t** planes, int32_t** eexp, const int32_t** order);
+                       int8_t** planes, int32_t** eexp);
 int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb,
                    const ctc_params* prm, const ctc_outputs* out, cudaStream_t st);
 
 // ---- FP64 path (ctc_local.cu) ----
+int fp64_tile_points(const LocalPlan& plan, int64_t n);
 int fp64_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb,
                      const ctc_params* prm, const ctc_outputs* out, cudaStream_t st);
 
 // per-point finalisation shared by the contraction kernels (ctc_local.cu)
 struct LocalSums;
+
+// d_sym of the density matrix now in d_D, on the stream.
+int set_symmetry_flag(ctc_molecule* mol, cudaStream_t st);
 
 // Host copy of D (internal order) brought up to date after a device-side
 // replacement (ctc_molecule_set_density_matrix); synchronises the device.
@@ -244,9 +252,6 @@ void destroy_esp(ctc_molecule* mol);
 // ---- adjoint (ctc_adjoint.cu) ----
 int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const double* v_rho,
                  const double* v_grad, double* dLdD, double* dLdR, cudaStream_t st);
-
-// chunk size (points) for a given AO footprint
-int64_t chunk_points(const ctc_molecule* mol, int nq_ao);
 
 // status word helpers: post_status enqueues the copy of the word after the
 // kernels just launched (no wait), poll_status reports a landed copy without

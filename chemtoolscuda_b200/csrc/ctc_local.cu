@@ -23,7 +23,8 @@
 //
 // Per chunk of tiles: screen -> AO block (compact) -> contraction + epilogue.
 // The FP64 contraction runs on the double-precision matrix units (mma.sync
-// m8n8k4 f64); the tensor-core split form is in ctc_tc.cu.
+// m8n8k4 f64, ctc_fp64.cuh); the tensor-core split form is in ctc_tc.cu.
+#include "ctc_fp64.cuh"
 #include "ctc_tiles.cuh"
 
 namespace ctc {
@@ -39,19 +40,22 @@ LocalPlan plan_local(const ctc_outputs* o) {
   return p;
 }
 
+// Points per tile of the FP64 form: 32 x 4 rows, or phi rows only: 128 points,
+// and 32 for calls whose 128-point tiles would leave SMs without work, up to
+// two 128-point tiles for every SM (density at 200 points of a 160-function
+// molecule: 58 us as two tiles of 128, 13 us as seven of 32).
+int fp64_tile_points(const LocalPlan& plan, int64_t n) {
+  return plan.nqa == 4 || n < (int64_t)128 * 148 * 2 ? 32 : 128;
+}
+
 int fp64_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb,
                      const ctc_params* prm, const ctc_outputs* out, cudaStream_t st) {
   if (tb.C <= 0) return CTC_OK;
-  int rc;
-  if (plan.nqa == 4) {
-    if ((rc = ensure_smem_attr((const void*)fp64_tile_kernel<4, 0>, (int)kSmemFp64)) != CTC_OK) return rc;
-    fp64_tile_kernel<4, 0><<<tb.C, kThreads, kSmemFp64, st>>>(tb, mol->d_D, mol->Mpad, *out, *prm, ForceArgs{});
-  } else {
-    if ((rc = ensure_smem_attr((const void*)fp64_tile_kernel<1, 0>, (int)kSmemFp64)) != CTC_OK) return rc;
-    fp64_tile_kernel<1, 0><<<tb.C, kThreads, kSmemFp64, st>>>(tb, mol->d_D, mol->Mpad, *out, *prm, ForceArgs{});
-  }
-  CTC_CUDA_TRY(cudaGetLastError());
-  return CTC_OK;
+  Fp64Args a{};
+  a.out = *out;
+  a.prm = *prm;
+  if (plan.nqa == 4) return launch_fp64<kFLocal4>(mol, tb, a, st);
+  return tb.TP == 32 ? launch_fp64<kFSmall1>(mol, tb, a, st) : launch_fp64<kFLocal1>(mol, tb, a, st);
 }
 
 int eval_local(ctc_molecule* mol, const PointSrc& src, int64_t n, int precision,
@@ -70,16 +74,15 @@ int eval_local(ctc_molecule* mol, const PointSrc& src, int64_t n, int precision,
   }
   // points per tile: 128 rows of the contraction (32 points x 4 quantities or
   // 128 points x phi)
-  const int TP = 128 / plan.nqa;
+  const int TP = precision == CTC_PREC_FP64 ? fp64_tile_points(plan, n) : 128 / plan.nqa;
   const int rows = TP * plan.nqa;
   // tensor-core path: the AO kernel also writes the int8 digit planes
   const std::function<int(const TileBatch&)> sliced_ao = [&](const TileBatch& tb) {
     int8_t* planes = nullptr;
     int32_t* eexp = nullptr;
-    const int32_t* order = nullptr;
-    int r = tc_slice_workspace(mol, tb, plan.nqa, st, &planes, &eexp, &order);
+    int r = tc_slice_workspace(mol, tb, plan.nqa, st, &planes, &eexp);
     if (r != CTC_OK) return r;
-    return launch_ao_tiles_sliced(mol, tb, plan.deriv, plan.nqa, planes, eexp, order, st);
+    return launch_ao_tiles_sliced(mol, tb, plan.deriv, plan.nqa, planes, eexp, tb.order, st);
   };
   int rc = run_tiles(
       mol, src, n, TP, plan.nq_ao, plan.deriv, st,

@@ -91,7 +91,7 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
   if (rc != CTC_OK) return rc;
 
   const LocalPlan plan = plan_local(out);
-  const int TP = 128 / plan.nqa;
+  const int TP = fp64_tile_points(plan, n);
   const int64_t ntiles = (n + TP - 1) / TP;
 
   // Morton order of the points over the molecule's box padded by 12 bohr,
@@ -157,6 +157,8 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
     tb.segs = tc.take<int32_t>((size_t)C * mol->nseg);
     tb.k0 = tc.take<int32_t>((size_t)C * mol->nseg);
     tb.aomap = tc.take<int32_t>((size_t)C * tb.Kcap);
+    tb.order = tc.take<int32_t>(C);
+    tb.counter = tc.take<int32_t>(1);
     tb.ao = tc.take<double>(ao_per_tile / sizeof(double) * (size_t)C);
     if (sort_end + tc.off > kNoAllocScratchBytes)
       return fail(CTC_ERR_INVALID, "ctc_eval_local_noalloc: internal scratch layout overflow");
@@ -173,12 +175,14 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
     const unsigned g = (unsigned)(((int64_t)tb.C * TP + 255) / 256);
     tile_gather_kernel<<<g, 256, 0, st>>>(d_points, perm, n, t0, tb);
     CTC_CUDA_TRY(cudaGetLastError());
-    screen_kernel<<<tb.C, kTileThreads, 0, st>>>(mol->d_segs, mol->nseg, tb, 128, mol->d_stats,
+    screen_kernel<<<tb.C, kTileThreads, 0, st>>>(mol->d_segs, mol->nseg, tb, TP * plan.nqa, mol->d_stats,
                                                  mol->d_status);
+    CTC_CUDA_TRY(cudaGetLastError());
+    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb);
     CTC_CUDA_TRY(cudaGetLastError());
     if ((rc = launch_ao_tiles(mol, tb, plan.deriv, st)) != CTC_OK) return rc;
     if ((rc = fp64_local_tiles(mol, plan, tb, prm, out, st)) != CTC_OK) return rc;
-    mol->host_launches += 4;
+    mol->host_launches += 5;
     mol->host_chunks += 1;
   }
   return CTC_OK;

@@ -46,11 +46,10 @@
 #include <cstdio>
 #include <cstdlib>
 
-#include <cub/device/device_radix_sort.cuh>
-
 #include "ctc_internal.h"
 #include "ctc_split.cuh"
 #include "ctc_finalize.cuh"
+#include "ctc_mbar.cuh"
 
 namespace ctc {
 
@@ -81,45 +80,6 @@ constexpr uint32_t kStatusTimeout = 0x7101;
 constexpr uint32_t kTileReaders = 6;
 
 // ------------------------------------------------------------------ PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}\n" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}\n" ::"r"(
-                   smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-// Bounded wait on an mbarrier phase: false once `limit` SM cycles have passed
-// (the pipeline's waits take the launch's limit, by default kWaitCycles).
-constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 1.9-2.0 GHz
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = kWaitCycles) {
-  const uint32_t a = smem_u32(bar);
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (clock64() - t0 > limit) return false;
-  }
-}
-
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }
@@ -962,27 +922,15 @@ int prepare_tc(ctc_molecule* mol, cudaStream_t st) {
 // Chunk workspace of the tensor-core path, one layout for both users (the AO
 // kernel that writes the digit planes and the contraction), for tiles of
 // `rows` operand rows (ctc_split.cuh):
-//   planes [C][rows / 128][5][128][Kcap] int8 | eexp [C][rows] | tile order:
-//   keys in/out, ids in, order [C] | tile counter | radix-sort temporary storage
+//   planes [C][rows / 128][5][128][Kcap] int8 | eexp [C][rows] | stage masks
 struct TcWorkspace {
   int8_t* planes;
   int32_t* eexp;
   uint32_t* mask;  // active K stages per tile (mask_words each), block-sparse D only
   int mask_words;
-  uint32_t* keys_in;
-  uint32_t* keys_out;
-  int32_t* ids;
-  int32_t* order;
-  int32_t* counter;
-  void* sort_tmp;
-  size_t sort_bytes;
 };
 
 int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t st, TcWorkspace* w) {
-  size_t sort_bytes = 0;
-  CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (uint32_t*)nullptr,
-                                               (uint32_t*)nullptr, (int32_t*)nullptr,
-                                               (int32_t*)nullptr, tb.C, 0, 15, st));
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -994,12 +942,6 @@ int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t 
   const int nbmax = tb.Kcap / kBK;
   const int mask_words = mol->d_nzpair ? (nbmax * nbmax + 31) / 32 : 0;
   const size_t o_mask = take(sizeof(uint32_t) * (size_t)tb.C * mask_words);
-  const size_t o_kin = take(sizeof(uint32_t) * tb.C);
-  const size_t o_kout = take(sizeof(uint32_t) * tb.C);
-  const size_t o_ids = take(sizeof(int32_t) * tb.C);
-  const size_t o_order = take(sizeof(int32_t) * tb.C);
-  const size_t o_counter = take(sizeof(int32_t));
-  const size_t o_tmp = take(sort_bytes);
   int rc = mol->ws_sl.ensure(off, st);
   if (rc != CTC_OK) return rc;
   char* base = (char*)mol->ws_sl.p;
@@ -1007,44 +949,16 @@ int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t 
   w->eexp = (int32_t*)(base + o_eexp);
   w->mask = mask_words ? (uint32_t*)(base + o_mask) : nullptr;
   w->mask_words = mask_words;
-  w->keys_in = (uint32_t*)(base + o_kin);
-  w->keys_out = (uint32_t*)(base + o_kout);
-  w->ids = (int32_t*)(base + o_ids);
-  w->order = (int32_t*)(base + o_order);
-  w->counter = (int32_t*)(base + o_counter);
-  w->sort_tmp = base + o_tmp;
-  w->sort_bytes = sort_bytes;
   return CTC_OK;
 }
 
-namespace {
-// sort keys: largest compact K first (ascending kMaxKt - kt), ids = tile index
-__global__ void tile_order_keys_kernel(const int32_t* __restrict__ kt, int C, uint32_t* keys,
-                                       int32_t* ids, int32_t* counter) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *counter = 0;
-  if (i < C) {
-    keys[i] = (uint32_t)(kMaxKt - min(kt[i], kMaxKt));
-    ids[i] = i;
-  }
-}
-}  // namespace
-
 int tc_slice_workspace(ctc_molecule* mol, const TileBatch& tb, int nqa, cudaStream_t st,
-                       int8_t** planes, int32_t** eexp, const int32_t** order) {
+                       int8_t** planes, int32_t** eexp) {
   TcWorkspace w;
   const int rc = tc_workspace(mol, tb, split_tile_rows(tb.TP, nqa), st, &w);
   if (rc != CTC_OK) return rc;
-  // the chunk's tile order, largest compact K first: the AO kernel's CTAs and
-  // the contraction's persistent CTAs both take the tiles in this order, so
-  // the last tiles of either launch are the cheapest ones
-  tile_order_keys_kernel<<<(tb.C + 255) / 256, 256, 0, st>>>(tb.kt, tb.C, w.keys_in, w.ids, w.counter);
-  CTC_CUDA_TRY(cudaGetLastError());
-  CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(w.sort_tmp, w.sort_bytes, w.keys_in, w.keys_out, w.ids,
-                                               w.order, tb.C, 0, 15, st));
   *planes = w.planes;
   *eexp = w.eexp;
-  *order = w.order;
   return CTC_OK;
 }
 
@@ -1055,9 +969,8 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
     return fail(CTC_ERR_UNSUPPORTED, "tensor-core split path: more than 16384 functions per tile");
   int rc = prepare_tc(mol, st);
   if (rc != CTC_OK) return rc;
-  // int8 planes of the tile rows, row exponents and the tile order (largest
-  // compact K first, zeroed tile counter), written for this chunk by
-  // tc_slice_workspace and the AO kernel (launch_ao_tiles_sliced)
+  // int8 planes of the tile rows and row exponents, written for this chunk by
+  // the AO kernel (launch_ao_tiles_sliced)
   if (!((plan.nqa == 4 && tb.TP == 32) || (plan.nqa == 1 && tb.TP == 128)))
     return fail(CTC_ERR_INVALID, "tensor-core split path: unsupported tile layout");
   const int rows = split_tile_rows(tb.TP, plan.nqa);
@@ -1089,8 +1002,8 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   a.out = *out;
   a.prm = *prm;
   a.status = mol->d_status;
-  a.order = w.order;
-  a.tile_counter = w.counter;
+  a.order = tb.order;
+  a.tile_counter = tb.counter;
   a.trace = nullptr;
   a.wait_cycles = mol->wait_cycles > 0 ? (long long)mol->wait_cycles : kWaitCycles;
   a.stage_mask = w.mask;

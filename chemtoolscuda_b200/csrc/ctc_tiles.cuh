@@ -400,258 +400,28 @@ __global__ void __launch_bounds__(kTileThreads)
   }
 }
 
-// ------------------------------------------------------------------ FP64 contraction kernel
-constexpr int BM = 128, BN = 64, BK = 32, STAGES = 3;
-constexpr int A_LD = BM + 4;  // A stage stored [k][row], 132 doubles: conflict-free fragment loads
-constexpr int B_LD = BN + 4;  // 68 doubles
-constexpr int C_LD = BN + 1;
-constexpr int A_STAGE = BK * A_LD, B_STAGE = BK * B_LD;
-constexpr int kThreads = 256;
-constexpr size_t kSmemPipe = sizeof(double) * STAGES * (A_STAGE + B_STAGE);
-constexpr size_t kSmemC = sizeof(double) * BM * C_LD;
-constexpr size_t kSmemFp64 = kSmemPipe > kSmemC ? kSmemPipe : kSmemC;
-static_assert(kKtAlign % BN == 0 && kKtAlign % BK == 0, "tile K alignment");
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  int sz = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  int sz = valid ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
-// One CTA per tile of PTS = 128/NQA points; tile row r holds quantity r / PTS
-// of point r % PTS (quantity 0 = phi, 1..3 = d_k phi).  It sweeps the tile's
-// compact nu range in 64-column slices, each with a full K loop over the
-// compact mu range (B = D gathered by index), and reduces every finished G
-// slice against the AO values of its columns.
-// Inputs of the force epilogue (EPI = 1): per-point dL/drho and dL/dgrad rho
-// indexed by the original point index, AO -> atom map, dL/dR accumulator.
-struct ForceArgs {
-  const double* v_rho = nullptr;
-  const double* v_grad = nullptr;
-  const int32_t* ao_atom = nullptr;
-  double* dLdR = nullptr;
-  int natom = 0;
-};
-constexpr int kMaxSmemAtoms = 1024;
-
-template <int NQA, int EPI>
-__global__ void __launch_bounds__(kThreads)
-    fp64_tile_kernel(TileBatch tb, const double* __restrict__ D, int Mpad, ctc_outputs out,
-                     ctc_params prm, ForceArgs fa) {
-  constexpr int PTS = BM / NQA;
-  constexpr int TPP = kThreads / PTS;  // epilogue threads per point
-  constexpr int NS = NQA == 4 ? 16 : 4;
-  extern __shared__ __align__(16) double smem[];
-  double* sA = smem;
-  double* sB = smem + STAGES * A_STAGE;
-  double* sC = smem;  // aliases the pipeline after the K loop
-  __shared__ int s_colmap[BN];
-  __shared__ double s_force[EPI == 1 ? 3 * kMaxSmemAtoms : 1];
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp & 3, wn = warp >> 2;
-  const int t = blockIdx.x;
-  const int kt = tb.kt[t];
-  const int nq_ao = tb.nq;
-  const int64_t ldq = (int64_t)PTS * tb.Kcap;  // stride between quantities
-  const double* A = tb.ao + (int64_t)t * nq_ao * ldq;
-  const int32_t* am = tb.aomap + (int64_t)t * tb.Kcap;
-
-  // epilogue ownership: lanes take consecutive points (coalesced AO reads),
-  // esub selects the column subset; partial sums meet in shared memory
-  const int epl = tid % PTS, esub = tid / PTS;
-  double acc_s[NS];
-#pragma unroll
-  for (int i = 0; i < NS; ++i) acc_s[i] = 0.0;
-  // force epilogue: per-point weights, per-CTA atom accumulators
-  const bool force_smem = EPI == 1 && fa.natom <= kMaxSmemAtoms;
-  double fvr = 0.0, fvg[3] = {0.0, 0.0, 0.0};
-  if constexpr (EPI == 1) {
-    for (int i = tid; i < 3 * fa.natom && force_smem; i += kThreads) s_force[i] = 0.0;
-    const int64_t oi = tb.out[(int64_t)t * PTS + epl];
-    if (oi >= 0) {
-      fvr = fa.v_rho[oi];
-      if (fa.v_grad)
-        for (int k = 0; k < 3; ++k) fvg[k] = fa.v_grad[3 * oi + k];
-    }
-  }
-
-  const int nkb = kt / BK;
-  for (int n0 = 0; n0 < kt; n0 += BN) {
-    if (tid < BN) s_colmap[tid] = am[n0 + tid];
-    __syncthreads();
-    double c[4][4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) c[i][j][0] = c[i][j][1] = 0.0;
-
-    auto load_stage = [&](int stage, int kb) {
-      double* a = sA + stage * A_STAGE;
-      double* b = sB + stage * B_STAGE;
-      const int k0 = kb * BK;
-      // A stage [k][row]: 32 k x 128 rows, each (q, k) a run of PTS points
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int ch = tid + i * kThreads;
-        const int kk = ch >> 6, r = (ch & 63) * 2;
-        const int q = r / PTS, pl = r % PTS;
-        cp_async16(a + kk * A_LD + r, A + q * ldq + (int64_t)(k0 + kk) * PTS + pl, true);
-      }
-      // B gather: 32 rows (compact mu) x 64 columns (compact nu), 8 bytes each
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int e = tid + i * kThreads;
-        const int r = e >> 6, cc = e & 63;
-        const int mu = am[k0 + r], nu = s_colmap[cc];
-        const bool v = mu >= 0 && nu >= 0;
-        cp_async8(b + r * B_LD + cc, D + (v ? (int64_t)mu * Mpad + nu : 0), v);
-      }
-    };
-
-    load_stage(0, 0);
-    cp_async_commit();
-    if (nkb > 1) load_stage(1, 1);
-    cp_async_commit();
-    for (int kb = 0; kb < nkb; ++kb) {
-      if (kb + 2 < nkb) load_stage((kb + 2) % STAGES, kb + 2);
-      cp_async_commit();
-      cp_async_wait<2>();
-      __syncthreads();
-      const double* a = sA + (kb % STAGES) * A_STAGE;
-      const double* b = sB + (kb % STAGES) * B_STAGE;
-#pragma unroll
-      for (int ks = 0; ks < BK; ks += 4) {
-        double af[4], bf[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          af[i] = a[(ks + (lane & 3)) * A_LD + wm * 32 + i * 8 + (lane >> 2)];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          bf[j] = b[(ks + (lane & 3)) * B_LD + wn * 32 + j * 8 + (lane >> 2)];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dmma(c[i][j][0], c[i][j][1], af[i], bf[j]);
-      }
-      __syncthreads();
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = wm * 32 + i * 8 + (lane >> 2);
-        const int cc = wn * 32 + j * 8 + 2 * (lane & 3);
-        sC[r * C_LD + cc] = c[i][j][0];
-        sC[r * C_LD + cc + 1] = c[i][j][1];
-      }
-    __syncthreads();
-    if constexpr (EPI == 0) {
-      {
-        // AO value of quantity q at column n0 + v for this point: A[q][n0 + v][epl]
-        const double* aop = A + (int64_t)n0 * PTS + epl;
-        for (int v = esub; v < BN; v += TPP) {
-          const double G0 = sC[(0 * PTS + epl) * C_LD + v];
-          const double phi = aop[v * PTS];
-          acc_s[0] += G0 * phi;
-          if (nq_ao >= 4) {
-            const double d0 = aop[ldq + v * PTS], d1 = aop[2 * ldq + v * PTS], d2 = aop[3 * ldq + v * PTS];
-            acc_s[1] += G0 * d0;
-            acc_s[2] += G0 * d1;
-            acc_s[3] += G0 * d2;
-            if constexpr (NQA == 4) {
-              const double G1 = sC[(1 * PTS + epl) * C_LD + v];
-              const double G2 = sC[(2 * PTS + epl) * C_LD + v];
-              const double G3 = sC[(3 * PTS + epl) * C_LD + v];
-              acc_s[10] += G1 * d0;
-              acc_s[11] += G1 * d1;
-              acc_s[12] += G1 * d2;
-              acc_s[13] += G2 * d1;
-              acc_s[14] += G2 * d2;
-              acc_s[15] += G3 * d2;
-              if (nq_ao == 10) {
-  #pragma unroll
-                for (int h = 0; h < 6; ++h) acc_s[4 + h] += G0 * aop[(4 + h) * ldq + v * PTS];
-              }
-            }
-          }
-        }
-      }
-    } else {
-      // dL/dR_A,j += sum over nu on atom A of
-      //   -2 v_rho d_j phi G0 - 2 sum_k v_k (d_j d_k phi G0 + d_j phi G_k)
-      const double* aop = A + (int64_t)n0 * PTS + epl;
-      const int hidx[3][3] = {{4, 5, 6}, {5, 7, 8}, {6, 8, 9}};
-      for (int v = esub; v < BN; v += TPP) {
-        const int nu = s_colmap[v];
-        if (nu < 0 || (fvr == 0.0 && fvg[0] == 0.0 && fvg[1] == 0.0 && fvg[2] == 0.0)) continue;
-        const int atom = fa.ao_atom[nu];
-        if (atom < 0) continue;
-        const double G0 = sC[(0 * PTS + epl) * C_LD + v];
-        double Gk[3] = {0.0, 0.0, 0.0};
-        if constexpr (NQA == 4) {
-          Gk[0] = sC[(1 * PTS + epl) * C_LD + v];
-          Gk[1] = sC[(2 * PTS + epl) * C_LD + v];
-          Gk[2] = sC[(3 * PTS + epl) * C_LD + v];
-        }
-        for (int j = 0; j < 3; ++j) {
-          const double dj = aop[(1 + j) * ldq + v * PTS];
-          double c = -2.0 * fvr * dj * G0;
-          if (fa.v_grad) {
-            for (int k = 0; k < 3; ++k)
-              c -= 2.0 * fvg[k] * (aop[hidx[j][k] * ldq + v * PTS] * G0 + dj * Gk[k]);
-          }
-          if (force_smem) atomicAdd(&s_force[3 * atom + j], c);
-          else atomicAdd(&fa.dLdR[3 * atom + j], c);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if constexpr (EPI == 1) {
-    __syncthreads();
-    if (force_smem)
-      for (int i = tid; i < 3 * fa.natom; i += kThreads)
-        if (s_force[i] != 0.0) atomicAdd(&fa.dLdR[i], s_force[i]);
-    return;
-  }
-  // sum the TPP column subsets of each point (sC is free after the last tile)
-  double* red = sC;
-#pragma unroll
-  for (int i = 0; i < NS; ++i) red[(esub * NS + i) * PTS + epl] = acc_s[i];
+// The chunk's tiles, largest compact set first (counting sort by kt / 64; the
+// order within a bin is free), and the chunk's tile counter set to zero.  Both
+// contractions and the tensor-core path's AO kernel take the tiles in this
+// order, so the last tiles of a launch are the cheapest.  One block: ~4 us at
+// 2 000 tiles, where a radix sort of the counts took ~8 us and two launches.
+constexpr int kOrderThreads = 1024;
+__global__ void __launch_bounds__(kOrderThreads) tile_order_kernel(TileBatch tb) {
+  using Scan = cub::BlockScan<int, kOrderThreads>;
+  __shared__ typename Scan::TempStorage tmp;
+  __shared__ int s_bin[kOrderThreads];
+  s_bin[threadIdx.x] = 0;
+  if (threadIdx.x == 0) *tb.counter = 0;
   __syncthreads();
-  const int64_t oidx = tb.out[(int64_t)t * PTS + epl];
-  if (esub == 0 && oidx >= 0 && !finite_point(tb.xyz + 3 * ((int64_t)t * PTS + epl))) {
-    nan_point(out, oidx);
-  } else if (esub == 0 && oidx >= 0) {
-    double s[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      double v = 0.0;
-      if (i < NS)
-        for (int e = 0; e < TPP; ++e) v += red[(e * NS + i) * PTS + epl];
-      s[i] = v;
-    }
-    finalize_point(s, NQA, nq_ao, out, oidx, prm);
-  }
+  auto bin = [&](int t) { return kOrderThreads - 1 - min(tb.kt[t] / kKtAlign, kOrderThreads - 1); };
+  for (int t = threadIdx.x; t < tb.C; t += kOrderThreads) atomicAdd(&s_bin[bin(t)], 1);
+  __syncthreads();
+  int first;
+  Scan(tmp).ExclusiveSum(s_bin[threadIdx.x], first);
+  __syncthreads();
+  s_bin[threadIdx.x] = first;
+  __syncthreads();
+  for (int t = threadIdx.x; t < tb.C; t += kOrderThreads) tb.order[atomicAdd(&s_bin[bin(t)], 1)] = t;
 }
 
 // ------------------------------------------------------------------ chunk scratch
@@ -680,6 +450,8 @@ size_t tile_bytes(const ctc_molecule* mol, int C, int TP, int Kcap_) {
   add(sizeof(int32_t) * (size_t)C * mol->nseg);
   add(sizeof(int32_t) * (size_t)C * mol->nseg);
   add(sizeof(int32_t) * (size_t)C * Kcap);
+  add(sizeof(int32_t) * C);
+  add(sizeof(int32_t));
   return b + 256;
 }
 
@@ -842,6 +614,8 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     tb.segs = cv.take<int32_t>((size_t)C * mol->nseg);
     tb.k0 = cv.take<int32_t>((size_t)C * mol->nseg);
     tb.aomap = cv.take<int32_t>((size_t)C * tb.Kcap);
+    tb.order = cv.take<int32_t>(C);
+    tb.counter = cv.take<int32_t>(1);
   }
   for (int64_t t0 = 0; t0 < ntiles; t0 += C) {
     tb.C = (int)std::min<int64_t>(C, ntiles - t0);
@@ -849,12 +623,14 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     screen_kernel<<<tb.C, kTileThreads, 0, st>>>(mol->d_segs, mol->nseg, tb, rows, mol->d_stats,
                                                  mol->d_status);
     CTC_CUDA_TRY(cudaGetLastError());
+    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb);
+    CTC_CUDA_TRY(cudaGetLastError());
     {
       ProfScope ps(mol, 1, st);
       rc = ao_launch ? (*ao_launch)(tb) : launch_ao_tiles(mol, tb, deriv, st);
       if (rc != CTC_OK) return rc;
     }
-    mol->host_launches += 3;
+    mol->host_launches += 4;
     mol->host_chunks += 1;
     if ((rc = compute(tb)) != CTC_OK) return rc;
   }

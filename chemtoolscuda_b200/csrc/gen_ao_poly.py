@@ -7,7 +7,10 @@ z, and the contracted radial sums R0, R1, R2 (see ctc_ao.cu).  With TRACK = 1
 the running maximum of the high word of |value| (sign cleared; its exponent is
 the exponent of the largest |value|) over the components is kept in mx[0], with
 TRACK = 4 also those of the three first derivatives in mx[1..3] (the row
-scales of the tensor-core split operands).  The terms come
+scales of the tensor-core split operands).  With TRACK = -1 the weighted row
+w = wv[0] value + wv[1..3] . gradient (the adjoint's second operand) is written
+as quantity 10, with TRACK = -2 the value and w (as quantity 1) are all that is
+written.  The terms come
 from gen_terms.py; writing their exponents as literals lets the compiler keep
 the power arrays in registers.
 
@@ -26,7 +29,7 @@ def emit_type(ti, l, pure):
            "template <int DERIV, int TRACK>",
            f"__device__ __forceinline__ void ao_poly_{ti}(const double* X, const double* Y, const double* Z,",
            "    double R0, double R1, double R2, double* __restrict__ o, int64_t ld_q, int64_t ldc, int nq_out,",
-           "    unsigned* mx) {"]
+           "    unsigned* mx, const double* wv) {"]
     for j, comp in enumerate(cs):
         out.append("  {")
         out.append("    double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0, q4 = 0.0, q5 = 0.0, q6 = 0.0, q7 = 0.0, q8 = 0.0, q9 = 0.0;")
@@ -49,7 +52,11 @@ def emit_type(ti, l, pure):
             out.append("    }")
         c = f"{j} * ldc"
         out.append(f"    o[{c}] = q0;")
-        out.append(f"    if (DERIV >= 1) {{ if (nq_out > 1) {{ o[ld_q + {c}] = q1; o[2 * ld_q + {c}] = q2; o[3 * ld_q + {c}] = q3; }} }}")
+        out.append("    if (TRACK < 0) {")
+        out.append("      const double w = wv[0] * q0 + wv[1] * q1 + wv[2] * q2 + wv[3] * q3;")
+        out.append(f"      o[(TRACK == -1 ? 10 : 1) * ld_q + {c}] = w;")
+        out.append("    }")
+        out.append(f"    if (TRACK != -2 && DERIV >= 1) {{ if (nq_out > 1) {{ o[ld_q + {c}] = q1; o[2 * ld_q + {c}] = q2; o[3 * ld_q + {c}] = q3; }} }}")
         out.append(f"    if (DERIV >= 2) {{ if (nq_out > 4) {{ o[4 * ld_q + {c}] = q4; o[5 * ld_q + {c}] = q5; o[6 * ld_q + {c}] = q6;")
         out.append(f"      o[7 * ld_q + {c}] = q7; o[8 * ld_q + {c}] = q8; o[9 * ld_q + {c}] = q9; }} }}")
         out.append("    if (TRACK >= 1) mx[0] = max(mx[0], abs_hi(q0));")
