@@ -12,15 +12,27 @@
 // depends on the point only through R, the Hermite densities h are built once
 // per molecule (host, all cores) and each point costs one Boys evaluation and
 // one R recursion per significant primitive pair -- no integral matrix.
-// Pairs are grouped by L = l_a + l_b; each class runs as its own kernel
-// (registers sized for its L), over a 2-D grid of 128-point blocks x slices
-// of the class's pairs.
+// Pairs are grouped by L = l_a + l_b into batches of one class.
+//
+// Far pairs.  Where every T = p |P - C|^2 of a block of points is beyond the
+// class's threshold, R^0_tuv is a derivative of sqrt(pi/p)/2 / |P - C| and the
+// pair is a point multipole:
+//     sum_tuv h_tuv R_tuv = ri H(x, y, z),  ri = 1/|P - C|, (x, y, z) = (P - C) ri^2,
+// H a polynomial of degree L with n_tuv(L) coefficients formed at set-up: one
+// reciprocal square root and one multiply-add per coefficient, instead of the R
+// recursion and a dot product (FP64 operations per pair and point for L = 0..4:
+// 12, 19, 25, 35, 50).  esp_far_kernel sums these pairs, all classes in one
+// launch, two points per thread.  Points are sorted along a Morton curve, so a
+// block's points lie close together and few pairs are near one of them and far
+// from the others.
+//
+// Near pairs of a block (a few per cent) go to esp_near_kernel: Boys function,
+// R recursion and the dot product with h, per point.
 //
 // Boys function F_n(T) (FP64): beyond a per-L threshold (T >= 38 + 3L, where
 // the neglected e^{-T} terms are below 2e-17 relative) the asymptotic forms
-// hold -- a far pair is a point multipole and costs one rsqrt and no
-// exponential; 99% of (point, pair) evaluations on molecular surfaces are of
-// this kind.  Below it, a 7-term Taylor expansion about the nearest point of
+// hold without an exponential; 99% of (point, pair) evaluations on molecular
+// surfaces are of this kind.  Below it, a 7-term Taylor expansion about the nearest point of
 // a 0.05-spaced table gives F_L, and F_{n-1} = (2T F_n + e^{-T})/(2n-1)
 // (downward recursion, stable) gives the rest.  The table is built at set-up
 // from the series F_m(T) = e^{-T} sum_i (2T)^i / ((2m+1)(2m+3)...(2m+2i+1)).
@@ -36,7 +48,7 @@
 #include <thread>
 #include <vector>
 
-#include "ctc_internal.h"
+#include "ctc_tiles.cuh"
 
 #define CTC_TERMS_HOST
 #include "ctc_terms.inc"
@@ -48,11 +60,10 @@ namespace {
 
 constexpr int kLmax = 8;                 // g x g
 constexpr int kTaylor = 7;               // terms of the Taylor expansion
-constexpr int kNF = kLmax + kTaylor;     // orders stored per table point
+constexpr int kRow = kTaylor + 1;         // table row: Taylor coefficients, e^{-T_i}
 constexpr double kTstep = 0.05;
 constexpr double kTmax = 64.0;           // table range: above every far_T(L <= 8)
 constexpr int kNT = (int)(kTmax / kTstep) + 2;
-constexpr double kPi = 3.14159265358979323846;
 
 __host__ __device__ constexpr int ntuv(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
 // index of (t,u,v): totals ascending; within a total s, t descending then u descending
@@ -65,15 +76,23 @@ __host__ __device__ constexpr int tuv_index(int t, int u, int v) {
 }
 
 struct EspPair {
-  double Px, Py, Pz, p;
-  double f0c;  // sqrt(pi / p) / 2: F_0 = f0c / |P - C| in the far field
+  double Px, Py, Pz;
+  double c0;    // constant coefficient of the far-field polynomial
+  double p;
+  double f0c;   // sqrt(pi / p) / 2: F_0 = f0c / |P - C| in the far field
+  double rfar;  // far field from this distance on: sqrt(far_T(L) / p)
   double pad;
 };
 struct EspBatch {
   int32_t b0, b1;   // pairs [b0, b1)
   int32_t h0;       // first Hermite coefficient
+  int32_t f0;       // first far-field coefficient (nfar(L) per pair)
   int32_t L;
+  int32_t pad[3];
 };
+// far-field coefficients of a pair besides the constant one, padded to whole
+// 16-byte loads
+__host__ __device__ constexpr int nfar(int L) { return ntuv(L) / 2 * 2; }
 
 double boys_series(int m, double T) {
   double term = 1.0 / (2 * m + 1), sum = term;
@@ -87,8 +106,8 @@ double boys_series(int m, double T) {
 
 }  // namespace
 
-// pairs per batch of class L: up to 256, with the batch's Hermite
-// coefficients within 32 KB (one barrier pair per batch in the class kernels)
+// pairs per batch of class L: up to 256, with the batch's coefficients within
+// 32 KB (a few barriers per batch)
 constexpr int kBatchPairs = 256;
 constexpr int kBatchH = 4096;
 __host__ __device__ constexpr int batch_pairs(int L) {
@@ -99,10 +118,11 @@ struct EspTables {
   double* d_boys = nullptr;
   EspPair* d_pairs = nullptr;
   double* d_h = nullptr;
+  double* d_far = nullptr;    // far-field polynomials, nfar(L) per pair
   EspBatch* d_batches = nullptr;
   double* d_atoms = nullptr;  // x y z Z per atom
   int npairs = 0, nbatch = 0, natom = 0;
-  int lb0[kLmax + 2] = {};  // batches of class L: [lb0[L], lb0[L + 1])
+  int Lmax = 0;  // largest class with pairs
   size_t nh = 0;
   // algorithmic FP64 work per point: sum over the kept pairs of
   // 2 n_tuv(L) (contraction) + 2 n_R(L) (R recursion) + 10 (L + 1) (Boys)
@@ -123,30 +143,41 @@ __host__ __device__ constexpr double far_T(int L) { return 38.0 + 3.0 * L; }
 // G_n = R^n_000 = (-2p)^n F_n(T), n = 0..L, at T = p r2.
 //  far field (T >= far_T(L)): the p dependence cancels except in F_0,
 //    G_0 = (sqrt(pi/p)/2) / r,  G_n = -(2n-1) G_{n-1} / r2  -- no exponential;
-//  otherwise: F_L from the 7-term Taylor table about the nearest 0.05 step,
+//  otherwise: F_L from the 7-term Taylor expansion about the nearest 0.05 step
+//    T_i (class L's table: coefficients F_{L+k}(T_i) / k! in d = T_i - T, then
+//    e^{-T_i}: one 64-byte row), e^{-T} = e^{-T_i} e^d with e^d by its series to
+//    d^7 (|d| <= 0.025: remainder below 4e-18),
 //    F_{n-1} = (2T F_n + e^{-T}) / (2n-1) downwards (stable for every T).
 template <int L>
 __device__ __forceinline__ void boys_g(double p, double f0c, double r2, const double* __restrict__ tab,
                                        double* G) {
   const double T = p * r2;
-  if (T >= far_T(L)) {
+  if (!(T < far_T(L))) {  // NaN too: its conversion to a table row is out of range
     const double ri = rsqrt(r2);
     const double ri2 = ri * ri;
     G[0] = f0c * ri;
 #pragma unroll
     for (int n = 1; n <= L; ++n) G[n] = -(double)(2 * n - 1) * ri2 * G[n - 1];
   } else {
-    const double e = exp(-T);
     const int i = __double2int_rn(T * (1.0 / kTstep));
-    const double d = i * kTstep - T;  // -(T - T_i)
-    const double* row = tab + i * kNF + L;
+    const double d = i * kTstep - T;  // T_i - T
+    const double2* row = reinterpret_cast<const double2*>(tab + ((int64_t)L * kNT + i) * kRow);
+    const double2 c01 = __ldg(row), c23 = __ldg(row + 1), c45 = __ldg(row + 2), c6e = __ldg(row + 3);
     double F[L + 1];
-    double fl = row[kTaylor - 1];
+    F[L] = fma(fma(fma(fma(fma(fma(c6e.x, d, c45.y), d, c45.x), d, c23.y), d, c23.x), d, c01.y), d, c01.x);
+    if (L > 0) {
+      double q = 1.0 / 5040.0;
+      q = fma(q, d, 1.0 / 720.0);
+      q = fma(q, d, 1.0 / 120.0);
+      q = fma(q, d, 1.0 / 24.0);
+      q = fma(q, d, 1.0 / 6.0);
+      q = fma(q, d, 0.5);
+      q = fma(q, d, 1.0);
+      q = fma(q, d, 1.0);
+      const double e = c6e.y * q, T2 = 2.0 * T;
 #pragma unroll
-    for (int k = kTaylor - 2; k >= 0; --k) fl = row[k] + fl * d * (1.0 / (double)(k + 1));
-    F[L] = fl;
-#pragma unroll
-    for (int n = L; n > 0; --n) F[n - 1] = (2.0 * T * F[n] + e) * (1.0 / (double)(2 * n - 1));
+      for (int n = L; n > 0; --n) F[n - 1] = fma(T2, F[n], e) * (1.0 / (double)(2 * n - 1));
+    }
     double m = 1.0;
 #pragma unroll
     for (int n = 0; n <= L; ++n) {
@@ -192,75 +223,326 @@ __device__ __forceinline__ void hermite_r(double X, double Y, double Z, const do
 
 constexpr int kEspThreads = 128;
 
-// Electronic ESP of the pairs of one angular class L: block (x, y) takes 128
-// points and slice y of the class's batches and writes its partial sum
-// sum_pairs sum_tuv h_tuv R_tuv (h already carries 2 pi / p) to row y of
-// part.  Rows are summed in a fixed order by esp_finish_kernel, so results do
-// not depend on the launch shape's timing.
-template <int L>
-__global__ void __launch_bounds__(kEspThreads)
-    esp_class_kernel(const EspPair* __restrict__ pairs, const double* __restrict__ hbuf,
-                     const EspBatch* __restrict__ batches, int b0, int nb, const double* __restrict__ tab,
-                     const double* __restrict__ pts, int64_t n, double* __restrict__ part) {
-  constexpr int NT = ntuv(L);
-  constexpr int BP = batch_pairs(L);
-  constexpr bool PAIRS2 = L <= 4;  // registers stay below ~170 up to L = 4
-  __shared__ EspPair sp[BP];
-  __shared__ double sh[BP * NT];
-  const int slices = gridDim.y, y = blockIdx.y;
-  const int bb = b0 + (int)((int64_t)nb * y / slices), be = b0 + (int)((int64_t)nb * (y + 1) / slices);
-  const int64_t ip = (int64_t)blockIdx.x * kEspThreads + threadIdx.x;
-  const bool live = ip < n;
-  double cx = 0, cy = 0, cz = 0;
-  if (live) {
-    cx = pts[3 * ip];
-    cy = pts[3 * ip + 1];
-    cz = pts[3 * ip + 2];
+// Points in their sorted order: xyz[3][n].
+__global__ void __launch_bounds__(256)
+    esp_gather_kernel(const double* __restrict__ pts, const int32_t* __restrict__ perm, int64_t n,
+                      double* __restrict__ xyz) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t p = perm ? perm[i] : i;
+  for (int d = 0; d < 3; ++d) xyz[d * n + i] = pts[3 * p + d];
+}
+
+// A point as the pair sums see it: finite coordinates are cut at 1e100 bohr, so
+// that |P - C|^2 stays finite (the potential there is zero to any precision).
+__device__ __forceinline__ double esp_coord(double v) {
+  return isfinite(v) ? fmin(fmax(v, -1e100), 1e100) : v;
+}
+
+// Sphere around the finite points of a block of kEspThreads threads with P
+// points each (centre of their box); radius -1e300 when no point is finite.
+template <int P>
+__device__ void esp_sphere(const double (*c)[3], const bool* live, double* ctr, double* rad) {
+  __shared__ double s_lo[3][kEspThreads / 32], s_hi[3][kEspThreads / 32], s_r[kEspThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int d = 0; d < 3; ++d) {
+    double lo = 1e300, hi = -1e300;
+    for (int p = 0; p < P; ++p)
+      if (live[p] && finite_point(c[p])) {
+        lo = fmin(lo, c[p][d]);
+        hi = fmax(hi, c[p][d]);
+      }
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
+      s_lo[d][warp] = lo;
+      s_hi[d][warp] = hi;
+    }
   }
-  double acc = 0.0;
+  __syncthreads();
+  bool any = false;
+  for (int d = 0; d < 3; ++d) {
+    double lo = 1e300, hi = -1e300;
+    for (int w = 0; w < kEspThreads / 32; ++w) {
+      lo = fmin(lo, s_lo[d][w]);
+      hi = fmax(hi, s_hi[d][w]);
+    }
+    any = lo <= hi;
+    ctr[d] = any ? 0.5 * lo + 0.5 * hi : 0.0;
+  }
+  double r2 = 0.0;
+  for (int p = 0; p < P; ++p)
+    if (live[p] && finite_point(c[p])) {
+      const double x = c[p][0] - ctr[0], y = c[p][1] - ctr[1], z = c[p][2] - ctr[2];
+      r2 = fmax(r2, x * x + y * y + z * z);
+    }
+  for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+  if (lane == 0) s_r[warp] = r2;
+  __syncthreads();
+  for (int w = 0; w < kEspThreads / 32; ++w) r2 = fmax(r2, s_r[w]);
+  *rad = any ? sqrt(r2) * (1.0 + 1e-12) + 1e-9 : -1e300;
+}
+
+// Indices of the batch's far (or near) pairs in order; returns their number.
+// The block's sphere decides, the same way in both kernels.
+template <bool FAR>
+__device__ int esp_select(const EspPair* __restrict__ pairs, int np, const double* ctr, double rad,
+                          uint16_t* s_list, int* s_cnt) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nch = (np + 31) / 32;
+  unsigned mask[kBatchPairs / kEspThreads];
+#pragma unroll
+  for (int k = 0; k < kBatchPairs / kEspThreads; ++k) {
+    const int ch = warp + k * (kEspThreads / 32), i = ch * 32 + lane;
+    bool take = false;
+    if (i < np) {
+      const EspPair& q = pairs[i];
+      const double x = q.Px - ctr[0], y = q.Py - ctr[1], z = q.Pz - ctr[2];
+      const double need = q.rfar + rad;
+      const bool far = need <= 0.0 || x * x + y * y + z * z >= need * need * (1.0 + 1e-12);
+      take = far == FAR;
+    }
+    mask[k] = __ballot_sync(0xffffffffu, take);
+    if (lane == 0 && ch < kBatchPairs / 32) s_cnt[ch] = ch < nch ? __popc(mask[k]) : 0;
+  }
+  __syncthreads();
+  int total = 0;
+#pragma unroll
+  for (int ch = 0; ch < kBatchPairs / 32; ++ch) total += s_cnt[ch];
+#pragma unroll
+  for (int k = 0; k < kBatchPairs / kEspThreads; ++k) {
+    const int ch = warp + k * (kEspThreads / 32);
+    int base = 0;
+    for (int j = 0; j < ch; ++j) base += s_cnt[j];
+    if ((mask[k] >> lane) & 1u) s_list[base + __popc(mask[k] & ((1u << lane) - 1u))] = (uint16_t)(ch * 32 + lane);
+  }
+  return total;
+}
+
+// 1 / sqrt(x): the hardware's approximation (relative error below 2^-19 over
+// the normal range) and one step of Householder's third-order iteration, whose
+// remainder is (5/16) e^3 < 2^-55 (measured: 1.4e-16; rsqrt(): 1.1e-16).
+__device__ __forceinline__ double esp_rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// acc[p] += ri H(x, y, z) of one far pair: nested Horner form, coefficients in
+// the order of their use (powers of x, then y, then z, descending; the constant
+// one is c0).
+template <int L, int P>
+__device__ __forceinline__ void esp_far_pair(const double4 q, const double2* __restrict__ h,
+                                             const double (*c)[3], double* acc) {
+  double x[P], y[P], z[P], ri[P];
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+    x[p] = q.x - c[p][0];
+    y[p] = q.y - c[p][1];
+    z[p] = q.z - c[p][2];
+    ri[p] = esp_rsqrt(x[p] * x[p] + y[p] * y[p] + z[p] * z[p]);
+    if (L == 1) {  // c0 + u (c . X): two operations fewer than scaling X
+      const double2 xy = h[0], zo = h[1];
+      const double s = fma(zo.x, z[p], fma(xy.y, y[p], xy.x * x[p]));
+      acc[p] = fma(ri[p], fma(ri[p] * ri[p], s, q.w), acc[p]);
+    } else if (L > 0) {
+      const double u = ri[p] * ri[p];
+      x[p] *= u;
+      y[p] *= u;
+      z[p] *= u;
+    }
+  }
+  if (L == 1) return;
+  double f[P], g[P], t[P];
+  int k = 0;
+#pragma unroll
+  for (int a = L; a >= 0; --a) {
+#pragma unroll
+    for (int b = L - a; b >= 0; --b) {
+#pragma unroll
+      for (int e = L - a - b; e >= 0; --e) {
+        const bool last = a == 0 && b == 0 && e == 0;
+        const double co = last ? q.w : ((k & 1) ? h[k >> 1].y : h[k >> 1].x);
+        ++k;
+#pragma unroll
+        for (int p = 0; p < P; ++p) t[p] = e == L - a - b ? co : fma(t[p], z[p], co);
+      }
+#pragma unroll
+      for (int p = 0; p < P; ++p) g[p] = b == L - a ? t[p] : fma(g[p], y[p], t[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) f[p] = a == L ? g[p] : fma(f[p], x[p], g[p]);
+  }
+#pragma unroll
+  for (int p = 0; p < P; ++p) acc[p] = fma(ri[p], f[p], acc[p]);
+}
+
+// Far pairs of block x's points (P per thread) in slice y of the batches of all
+// classes: row y of part.  Rows are summed in a fixed order by
+// esp_finish_kernel, so results do not depend on timing.
+// Bound: FP64 pipe.  100 atoms (1 604 functions, 8e5 pairs), 1e5 surface
+// points: the five class kernels with the R recursion took 287 ms.
+template <int P>
+__global__ void __launch_bounds__(kEspThreads)
+    esp_far_kernel(const EspPair* __restrict__ pairs, const double* __restrict__ far,
+                   const EspBatch* __restrict__ batches, int nb, const double* __restrict__ xyz, int64_t n,
+                   double* __restrict__ part) {
+  __shared__ double4 sp[kBatchPairs];
+  __shared__ __align__(16) double sh[kBatchH];
+  __shared__ uint16_t s_list[kBatchPairs];
+  __shared__ int s_cnt[kBatchPairs / 32];
+  const int slices = gridDim.y, y = blockIdx.y;
+  const int bb = (int)((int64_t)nb * y / slices), be = (int)((int64_t)nb * (y + 1) / slices);
+  double c[P][3], acc[P];
+  bool live[P];
+  int64_t ip[P];
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+    ip[p] = ((int64_t)blockIdx.x * P + p) * kEspThreads + threadIdx.x;
+    live[p] = ip[p] < n;
+    for (int d = 0; d < 3; ++d) c[p][d] = esp_coord(xyz[d * n + (live[p] ? ip[p] : n - 1)]);
+    acc[p] = 0.0;
+  }
+  double ctr[3], rad;
+  esp_sphere<P>(c, live, ctr, &rad);
   for (int b = bb; b < be; ++b) {
     const EspBatch bt = batches[b];
     const int np = bt.b1 - bt.b0;
+    __syncthreads();  // readers of the previous batch are done
+    for (int i = threadIdx.x; i < np; i += kEspThreads) {
+      const EspPair& q = pairs[bt.b0 + i];
+      sp[i] = make_double4(q.Px, q.Py, q.Pz, q.c0);
+    }
+    const int nd = np * nfar(bt.L) / 2;
+    const double2* src = reinterpret_cast<const double2*>(far + bt.f0);
+    for (int i = threadIdx.x; i < nd; i += kEspThreads) reinterpret_cast<double2*>(sh)[i] = src[i];
+    const int nf = esp_select<true>(pairs + bt.b0, np, ctr, rad, s_list, s_cnt);
     __syncthreads();
-    for (int i = threadIdx.x; i < np; i += kEspThreads) sp[i] = pairs[bt.b0 + i];
-    for (int i = threadIdx.x; i < np * NT; i += kEspThreads) sh[i] = hbuf[bt.h0 + i];
-    __syncthreads();
-    if (!live) continue;
-    auto pair_sum = [&](int i) -> double {
-      const EspPair q = sp[i];
-      const double X = q.Px - cx, Y = q.Py - cy, Z = q.Pz - cz;
-      double G[L + 1];
-      boys_g<L>(q.p, q.f0c, X * X + Y * Y + Z * Z, tab, G);
-      double R[NT];
-      hermite_r<L>(X, Y, Z, G, R);
-      const double* h = sh + i * NT;
-      double s = 0.0;
+#define CTC_ESP_FAR(LL)                                                                                \
+  case LL:                                                                                             \
+    for (int k = 0; k < nf; ++k) {                                                                     \
+      const int i = s_list[k];                                                                         \
+      esp_far_pair<LL, P>(sp[i], reinterpret_cast<const double2*>(sh) + i * (nfar(LL) / 2), c, acc);   \
+    }                                                                                                  \
+    break;
+    switch (bt.L) {
+      CTC_ESP_FAR(0)
+      CTC_ESP_FAR(1)
+      CTC_ESP_FAR(2)
+      CTC_ESP_FAR(3)
+      CTC_ESP_FAR(4)
+      CTC_ESP_FAR(5)
+      CTC_ESP_FAR(6)
+      CTC_ESP_FAR(7)
+      CTC_ESP_FAR(8)
+    }
+#undef CTC_ESP_FAR
+  }
 #pragma unroll
-      for (int k = 0; k < NT; ++k) s += h[k] * R[k];
-      return s;
-    };
-    int i = 0;
-    if (PAIRS2) {
-      // two pairs per iteration: two independent dependency chains (Boys, R
-      // recursion, dot product) for the FP64 pipe; added in pair order
-      for (; i + 1 < np; i += 2) {
-        const double s0 = pair_sum(i), s1 = pair_sum(i + 1);
-        acc += s0;
-        acc += s1;
+  for (int p = 0; p < P; ++p)
+    if (live[p]) part[(int64_t)y * n + ip[p]] = acc[p];
+}
+
+// Near pairs of the same blocks and slices.  A warp whose points are all far
+// from the pair takes the far-field polynomial, the others the Boys function
+// and the R recursion (far points of such a warp by the asymptotic form).
+// LMAX bounds the classes (the R recursion's registers).
+template <int LMAX, int P>
+__global__ void __launch_bounds__(kEspThreads)
+    esp_near_kernel(const EspPair* __restrict__ pairs, const double* __restrict__ hbuf,
+                    const double* __restrict__ far, const EspBatch* __restrict__ batches, int nb, const double* __restrict__ tab,
+                    const double* __restrict__ xyz, int64_t n, double* __restrict__ part) {
+  __shared__ EspPair sp[kBatchPairs / 4];
+  __shared__ double sh[kBatchH / 4];
+  __shared__ __align__(16) double sf[kBatchH / 4];
+  __shared__ uint16_t s_list[kBatchPairs];
+  __shared__ int s_cnt[kBatchPairs / 32];
+  const int slices = gridDim.y, y = blockIdx.y;
+  const int bb = (int)((int64_t)nb * y / slices), be = (int)((int64_t)nb * (y + 1) / slices);
+  double c[P][3], acc[P];
+  bool live[P];
+  int64_t ip[P];
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+    ip[p] = ((int64_t)blockIdx.x * P + p) * kEspThreads + threadIdx.x;
+    live[p] = ip[p] < n;
+    for (int d = 0; d < 3; ++d) c[p][d] = esp_coord(xyz[d * n + (live[p] ? ip[p] : n - 1)]);
+    acc[p] = 0.0;
+  }
+  double ctr[3], rad;
+  esp_sphere<P>(c, live, ctr, &rad);
+  for (int b = bb; b < be; ++b) {
+    const EspBatch bt = batches[b];
+    __syncthreads();
+    const int nn = esp_select<false>(pairs + bt.b0, bt.b1 - bt.b0, ctr, rad, s_list, s_cnt);
+    // the near pairs in groups that fit the shared arrays
+    const int NT = ntuv(bt.L), cap = min(kBatchPairs, kBatchH / NT) / 4;
+    for (int g0 = 0; g0 < nn; g0 += cap) {
+      const int ng = min(cap, nn - g0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < ng; i += kEspThreads) sp[i] = pairs[bt.b0 + s_list[g0 + i]];
+      for (int i = threadIdx.x; i < ng * NT; i += kEspThreads)
+        sh[i] = hbuf[bt.h0 + (int64_t)s_list[g0 + i / NT] * NT + i % NT];
+      const int NF = nfar(bt.L);
+      for (int i = threadIdx.x; i < ng * NF; i += kEspThreads)
+        sf[i] = far[bt.f0 + (int64_t)s_list[g0 + i / NF] * NF + i % NF];
+      __syncthreads();
+      auto run = [&](auto lc) {
+        constexpr int L = decltype(lc)::value;
+        if constexpr (L <= LMAX) {
+          for (int k = 0; k < ng; ++k) {
+            const EspPair q = sp[k];
+            const double* h = sh + k * ntuv(L);
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+              const double X = q.Px - c[p][0], Y = q.Py - c[p][1], Z = q.Pz - c[p][2];
+              const double r2 = X * X + Y * Y + Z * Z;
+              if (__all_sync(0xffffffffu, q.p * r2 >= far_T(L))) {
+                esp_far_pair<L, 1>(make_double4(q.Px, q.Py, q.Pz, q.c0),
+                                   reinterpret_cast<const double2*>(sf) + k * (nfar(L) / 2), c + p, acc + p);
+                continue;
+              }
+              double G[L + 1];
+              boys_g<L>(q.p, q.f0c, r2, tab, G);
+              double R[ntuv(L)];
+              hermite_r<L>(X, Y, Z, G, R);
+              double s = 0.0;
+#pragma unroll
+              for (int j = 0; j < ntuv(L); ++j) s += h[j] * R[j];
+              acc[p] += s;
+            }
+          }
+        }
+      };
+      switch (bt.L) {
+        case 0: run(std::integral_constant<int, 0>{}); break;
+        case 1: run(std::integral_constant<int, 1>{}); break;
+        case 2: run(std::integral_constant<int, 2>{}); break;
+        case 3: run(std::integral_constant<int, 3>{}); break;
+        case 4: run(std::integral_constant<int, 4>{}); break;
+        case 5: run(std::integral_constant<int, 5>{}); break;
+        case 6: run(std::integral_constant<int, 6>{}); break;
+        case 7: run(std::integral_constant<int, 7>{}); break;
+        default: run(std::integral_constant<int, 8>{}); break;
       }
     }
-    for (; i < np; ++i) acc += pair_sum(i);
   }
-  if (live) part[(int64_t)y * n + ip] = acc;
+#pragma unroll
+  for (int p = 0; p < P; ++p)
+    if (live[p]) part[(int64_t)y * n + ip[p]] = acc[p];
 }
 
 // V = sum_A Z_A / |C - R_A| - (sum of the rows of part, in row order).
 __global__ void __launch_bounds__(256)
     esp_finish_kernel(const double* __restrict__ part, int rows, const double* __restrict__ atoms, int natom,
-                      const double* __restrict__ pts, int64_t n, double* __restrict__ out) {
+                      const double* __restrict__ xyz, const int32_t* __restrict__ perm, int64_t n,
+                      double* __restrict__ out) {
   const int64_t ip = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (ip >= n) return;
-  const double cx = pts[3 * ip], cy = pts[3 * ip + 1], cz = pts[3 * ip + 2];
+  const double cx = xyz[ip], cy = xyz[n + ip], cz = xyz[2 * n + ip];
   double elec = 0.0;
   for (int r = 0; r < rows; ++r) elec += part[(int64_t)r * n + ip];
   double nuc = 0.0;
@@ -268,7 +550,7 @@ __global__ void __launch_bounds__(256)
     const double dx = cx - atoms[4 * a], dy = cy - atoms[4 * a + 1], dz = cz - atoms[4 * a + 2];
     nuc += atoms[4 * a + 3] / sqrt(dx * dx + dy * dy + dz * dz);
   }
-  out[ip] = nuc - elec;
+  out[perm ? perm[ip] : ip] = nuc - elec;
 }
 
 // ------------------------------------------------------------------ host side
@@ -322,6 +604,62 @@ struct PairOut {
   std::vector<double> h;
 };
 
+// Far-field polynomial of a pair.  d_x^t d_y^u d_z^v (1/r) = Q_tuv r^(-2l-1),
+// l = t + u + v, with Q_000 = 1 and Q_{t+1,u,v} = r^2 d_x Q - (2l+1) x Q (the
+// same for y, z): homogeneous of degree l with integer coefficients.  With
+// (x, y, z) scaled by 1/r^2, sum_tuv h_tuv Q_tuv r^(-2l-1) is 1/r times one
+// polynomial of degree L.
+struct FarTerms {
+  // q[tuv]: coefficients of Q_tuv by tuv_index of the monomial's exponents,
+  // from the first monomial of its degree
+  std::vector<std::vector<double>> q;
+  FarTerms() : q(ntuv(kLmax)) {
+    q[0] = {1.0};
+    for (int s = 1; s <= kLmax; ++s)
+      for (int t = s; t >= 0; --t)
+        for (int u = s - t; u >= 0; --u) {
+          const int e[3] = {t, u, s - t - u};
+          const int ax = e[0] ? 0 : (e[1] ? 1 : 2);
+          int low[3] = {e[0], e[1], e[2]};
+          --low[ax];
+          const int l = s - 1, base_l = ntuv(l - 1), base_s = ntuv(s - 1);
+          const std::vector<double>& ql = q[tuv_index(low[0], low[1], low[2])];
+          std::vector<double> r(ntuv(s) - base_s, 0.0);
+          for (int a = 0; a <= l; ++a)
+            for (int b = 0; a + b <= l; ++b) {
+              const int m[3] = {a, b, l - a - b};
+              const double c = ql[tuv_index(m[0], m[1], m[2]) - base_l];
+              if (c == 0.0) continue;
+              auto add = [&](int d0, int d1, int d2, double v) {
+                r[tuv_index(m[0] + d0, m[1] + d1, m[2] + d2) - base_s] += v;
+              };
+              add(ax == 0, ax == 1, ax == 2, -(2.0 * l + 1.0) * c);
+              if (m[ax] > 0)
+                for (int k = 0; k < 3; ++k)
+                  add(2 * (k == 0) - (ax == 0), 2 * (k == 1) - (ax == 1), 2 * (k == 2) - (ax == 2), m[ax] * c);
+            }
+          q[tuv_index(t, u, s - t - u)] = std::move(r);
+        }
+  }
+  // coefficients in Horner order, times f0c; returns the constant one
+  double of(int L, const double* h, double f0c, double* out) const {
+    double poly[ntuv(kLmax)] = {};
+    for (int i = 0, s = 0; i < ntuv(L); ++i) {
+      if (i == ntuv(s)) ++s;
+      if (h[i] == 0.0) continue;
+      const int base = ntuv(s - 1);
+      for (size_t m = 0; m < q[i].size(); ++m) poly[base + m] += h[i] * q[i][m];
+    }
+    int k = 0;
+    for (int a = L; a >= 0; --a)
+      for (int b = L - a; b >= 0; --b)
+        for (int c = L - a - b; c >= 0; --c)
+          if (a || b || c) out[k++] = f0c * poly[tuv_index(a, b, c)];
+    while (k < nfar(L)) out[k++] = 0.0;
+    return f0c * poly[0];
+  }
+};
+
 // Upper bound of |R^0_tuv(p, X)| over all points for t + u + v = s, used to
 // bound a pair's contribution: (2p)^(s/2) times a generous constant in s.
 inline double r_bound(double p, int s) { return std::pow(2.0 * p + 1.0, 0.5 * s) * std::pow(3.0, s); }
@@ -333,6 +671,7 @@ void destroy_esp(ctc_molecule* mol) {
   cudaFree(mol->esp->d_boys);
   cudaFree(mol->esp->d_pairs);
   cudaFree(mol->esp->d_h);
+  cudaFree(mol->esp->d_far);
   cudaFree(mol->esp->d_batches);
   cudaFree(mol->esp->d_atoms);
   delete mol->esp;
@@ -398,8 +737,8 @@ static int build_esp(ctc_molecule* mol) {
             hermite_e(A.l, B.l, a, b, ZAB, Ez);
             PairOut po;
             po.L = L;
-            po.pr = {(a * A.cx + b * B.cx) / p, (a * A.cy + b * B.cy) / p, (a * A.cz + b * B.cz) / p, p,
-                     0.5 * std::sqrt(kPi / p), 0.0};
+            po.pr = {(a * A.cx + b * B.cx) / p, (a * A.cy + b * B.cy) / p, (a * A.cz + b * B.cz) / p, 0.0, p,
+                     0.5 * std::sqrt(kPi / p), std::sqrt(far_T(L) / p), 0.0};
             po.h.assign(NT, 0.0);
             const int LB1 = B.l + 1, L1 = L + 1;
             for (int ma = 0; ma < mA; ++ma) {
@@ -466,29 +805,44 @@ static int build_esp(ctc_molecule* mol) {
   }
   // gather, sorted by L, into batches of equal L
   std::vector<EspPair> pairs;
-  std::vector<double> hv;
+  std::vector<double> hv, fv;
   std::vector<EspBatch> batches;
-  int lb0[kLmax + 2] = {};
+  int Lmax = 0;
+  static const FarTerms far_terms;
   for (int L = 0; L <= kLmax; ++L) {
     const int per = batch_pairs(L);
-    lb0[L] = (int)batches.size();
     int in_batch = 0;
     for (auto& o : outs)
       for (auto& po : o) {
         if (po.L != L) continue;
-        if (in_batch == 0) batches.push_back({(int32_t)pairs.size(), (int32_t)pairs.size(), (int32_t)hv.size(), L});
+        Lmax = L;
+        if (in_batch == 0)
+          batches.push_back({(int32_t)pairs.size(), (int32_t)pairs.size(), (int32_t)hv.size(), (int32_t)fv.size(), L, {0, 0, 0}});
+        double fc[ntuv(kLmax) + 1];
+        po.pr.c0 = far_terms.of(L, po.h.data(), po.pr.f0c, fc);
+        fv.insert(fv.end(), fc, fc + nfar(L));
         pairs.push_back(po.pr);
         hv.insert(hv.end(), po.h.begin(), po.h.end());
         batches.back().b1 = (int32_t)pairs.size();
         if (++in_batch == per) in_batch = 0;
       }
   }
-  lb0[kLmax + 1] = (int)batches.size();
   if (hv.size() > (size_t)INT32_MAX) return fail(CTC_ERR_UNSUPPORTED, "ESP: too many pair coefficients");
   // Boys table
-  std::vector<double> tab((size_t)kNT * kNF);
-  for (int i = 0; i < kNT; ++i)
-    for (int m = 0; m < kNF; ++m) tab[(size_t)i * kNF + m] = boys_series(m, i * kTstep);
+  std::vector<double> tab((size_t)(kLmax + 1) * kNT * kRow);
+  for (int i = 0; i < kNT; ++i) {
+    double F[kLmax + kTaylor];
+    for (int m = 0; m < kLmax + kTaylor; ++m) F[m] = boys_series(m, i * kTstep);
+    for (int L = 0; L <= kLmax; ++L) {
+      double* row = &tab[((size_t)L * kNT + i) * kRow];
+      double fact = 1.0;
+      for (int k = 0; k < kTaylor; ++k) {
+        row[k] = F[L + k] / fact;
+        fact *= k + 1;
+      }
+      row[kTaylor] = std::exp(-i * kTstep);
+    }
+  }
   std::vector<double> atoms(4 * (size_t)std::max(mol->natom, 1));
   for (int a = 0; a < mol->natom; ++a) {
     atoms[4 * a] = mol->atom_xyz[3 * a];
@@ -506,7 +860,7 @@ static int build_esp(ctc_molecule* mol) {
     e->mean_L += (double)np * bt.L;
   }
   if (!pairs.empty()) e->mean_L /= (double)pairs.size();
-  std::copy(lb0, lb0 + kLmax + 2, e->lb0);
+  e->Lmax = Lmax;
   e->npairs = (int)pairs.size();
   e->nbatch = (int)batches.size();
   e->natom = mol->natom;
@@ -521,6 +875,7 @@ static int build_esp(ctc_molecule* mol) {
   if ((rc = up((void**)&e->d_boys, tab.data(), tab.size() * sizeof(double))) ||
       (rc = up((void**)&e->d_pairs, pairs.empty() ? nullptr : pairs.data(), pairs.size() * sizeof(EspPair))) ||
       (rc = up((void**)&e->d_h, hv.empty() ? nullptr : hv.data(), hv.size() * sizeof(double))) ||
+      (rc = up((void**)&e->d_far, fv.empty() ? nullptr : fv.data(), fv.size() * sizeof(double))) ||
       (rc = up((void**)&e->d_batches, batches.empty() ? nullptr : batches.data(), batches.size() * sizeof(EspBatch))) ||
       (rc = up((void**)&e->d_atoms, atoms.data(), atoms.size() * sizeof(double)))) {
     destroy_esp(mol);
@@ -559,47 +914,61 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
   constexpr int64_t kChunk = (int64_t)1 << 22;
   for (int64_t p0 = 0; p0 < n; p0 += kChunk) {
     const int64_t m = std::min(kChunk, n - p0);
-    const int64_t gx = (m + kEspThreads - 1) / kEspThreads;
-    // slices of each class's batches: about 8 blocks per SM in every class kernel
-    int sl[kLmax + 1], rows = 0;
-    for (int L = 0; L <= kLmax; ++L) {
-      const int nb = e->lb0[L + 1] - e->lb0[L];
-      const int64_t want = (8 * (int64_t)nsm + gx - 1) / gx;
-      sl[L] = nb == 0 ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)nb, 65535}));
-      rows += sl[L];
-    }
-    if (int rc = mol->ws_esp.ensure(sizeof(double) * std::max<int64_t>(1, (int64_t)rows * m), st); rc != CTC_OK)
-      return rc;
-    double* part = (double*)mol->ws_esp.p;
     const double* pts = d_points + 3 * p0;
-    int r = 0;
-    for (int L = 0; L <= kLmax; ++L) {
-      if (!sl[L]) continue;
-      const dim3 grid((unsigned)gx, (unsigned)sl[L]);
-      const int b0 = e->lb0[L], nb = e->lb0[L + 1] - e->lb0[L];
-      double* pr = part + (int64_t)r * m;
-#define CTC_ESP_CLASS(LL)                                                                                   \
-  case LL:                                                                                                  \
-    esp_class_kernel<LL><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_batches, b0, nb, e->d_boys, \
-                                                      pts, m, pr);                                         \
-    break;
-      switch (L) {
-        CTC_ESP_CLASS(0)
-        CTC_ESP_CLASS(1)
-        CTC_ESP_CLASS(2)
-        CTC_ESP_CLASS(3)
-        CTC_ESP_CLASS(4)
-        CTC_ESP_CLASS(5)
-        CTC_ESP_CLASS(6)
-        CTC_ESP_CLASS(7)
-        CTC_ESP_CLASS(8)
-      }
-#undef CTC_ESP_CLASS
+    // two points per thread share a pair's coefficients; one when the points
+    // would fill less than a block per SM (the pairs are then cut into more
+    // slices) or the R recursion of classes above 4 needs all registers
+    const int P = e->Lmax <= 4 && m >= (int64_t)2 * kEspThreads * nsm ? 2 : 1;
+    const int64_t gx = (m + P * kEspThreads - 1) / (P * kEspThreads);
+    // slices of the batches: about 32 blocks per SM, at least a batch each
+    const int64_t want = (32 * (int64_t)nsm + gx - 1) / gx;
+    const int S = e->nbatch == 0 ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)e->nbatch, 65535}));
+    const bool sort = m > kEspThreads;
+    size_t tmp_bytes = 0;
+    if (sort)
+      CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                                   (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, kMortonSortBits, st));
+    const size_t need = sizeof(double) * (size_t)(2 * S + 3) * m + 4 * sizeof(int32_t) * (size_t)m + tmp_bytes + 4096;
+    if (int rc = mol->ws_esp.ensure(need, st); rc != CTC_OK) return rc;
+    Carve cv{(char*)mol->ws_esp.p};
+    double* part = cv.take<double>((size_t)std::max(1, 2 * S) * m);
+    double* xyz = cv.take<double>(3 * (size_t)m);
+    int32_t* perm = nullptr;
+    const unsigned g = (unsigned)((m + 255) / 256);
+    if (sort) {
+      uint32_t* k_in = cv.take<uint32_t>(m);
+      uint32_t* k_out = cv.take<uint32_t>(m);
+      int32_t* v_in = cv.take<int32_t>(m);
+      perm = cv.take<int32_t>(m);
+      void* tmp = cv.take<char>(tmp_bytes);
+      double lo[3], ext = 0;
+      morton_box(mol, lo, &ext);
+      morton_kernel<<<g, 256, 0, st>>>(pts, m, lo[0], lo[1], lo[2], 1024.0 / ext, k_in, v_in);
       CTC_CUDA_TRY(cudaGetLastError());
-      r += sl[L];
+      CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k_in, k_out, v_in, perm, (int)m, 0,
+                                                   kMortonSortBits, st));
     }
-    esp_finish_kernel<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(part, rows, e->d_atoms, e->natom, pts, m,
-                                                                   d_out + p0);
+    esp_gather_kernel<<<g, 256, 0, st>>>(pts, perm, m, xyz);
+    CTC_CUDA_TRY(cudaGetLastError());
+    if (S > 0) {
+      const dim3 grid((unsigned)gx, (unsigned)S);
+      double* near = part + (int64_t)S * m;
+      if (P == 2) esp_far_kernel<2><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_far, e->d_batches, e->nbatch, xyz, m, part);
+      else esp_far_kernel<1><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_far, e->d_batches, e->nbatch, xyz, m, part);
+      CTC_CUDA_TRY(cudaGetLastError());
+#define CTC_ESP_NEAR(LM, PP)                                                                                       \
+  esp_near_kernel<LM, PP><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch,      \
+                                                       e->d_boys, xyz, m, near)
+      if (e->Lmax > 6) CTC_ESP_NEAR(8, 1);
+      else if (e->Lmax > 4) CTC_ESP_NEAR(6, 1);
+      else if (e->Lmax > 2 && P == 2) CTC_ESP_NEAR(4, 2);
+      else if (e->Lmax > 2) CTC_ESP_NEAR(4, 1);
+      else if (P == 2) CTC_ESP_NEAR(2, 2);
+      else CTC_ESP_NEAR(2, 1);
+#undef CTC_ESP_NEAR
+      CTC_CUDA_TRY(cudaGetLastError());
+    }
+    esp_finish_kernel<<<g, 256, 0, st>>>(part, 2 * S, e->d_atoms, e->natom, xyz, perm, m, d_out + p0);
     CTC_CUDA_TRY(cudaGetLastError());
   }
   return CTC_OK;

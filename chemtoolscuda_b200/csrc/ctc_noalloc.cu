@@ -96,20 +96,8 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
 
   // Morton order of the points over the molecule's box padded by 12 bohr,
   // the same ordering ctc_eval_local uses.
-  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  for (int a = 0; a < mol->natom; ++a)
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = std::min(lo[d], mol->atom_xyz[3 * a + d]);
-      hi[d] = std::max(hi[d], mol->atom_xyz[3 * a + d]);
-    }
-  if (mol->natom == 0)
-    for (int d = 0; d < 3; ++d) { lo[d] = -1; hi[d] = 1; }
-  double ext = 0;
-  for (int d = 0; d < 3; ++d) {
-    lo[d] -= 12.0;
-    hi[d] += 12.0;
-    ext = std::max(ext, hi[d] - lo[d]);
-  }
+  double lo[3], ext = 0;
+  morton_box(mol, lo, &ext);
   size_t sort_tmp = 0;
   CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_tmp, (uint32_t*)nullptr,
                                                (uint32_t*)nullptr, (int32_t*)nullptr,

@@ -75,6 +75,21 @@ __global__ void morton_kernel(const double* __restrict__ pts, int64_t n, double 
   vals[i] = (int32_t)i;
 }
 
+// Corner and edge of the cube the Morton keys cover: the molecule's box padded
+// by 12 bohr.
+inline void morton_box(const ctc_molecule* mol, double* lo, double* ext) {
+  *ext = 24.0;
+  for (int d = 0; d < 3; ++d) {
+    double a = mol->natom ? 1e300 : -1.0, b = mol->natom ? -1e300 : 1.0;
+    for (int i = 0; i < mol->natom; ++i) {
+      a = std::min(a, mol->atom_xyz[3 * i + d]);
+      b = std::max(b, mol->atom_xyz[3 * i + d]);
+    }
+    lo[d] = a - 12.0;
+    *ext = std::max(*ext, b - a + 24.0);
+  }
+}
+
 // Sort-tile-recursive packing of explicit points (Leutenegger, Lopez and
 // Edgington, "STR: a simple and efficient algorithm for R-tree packing",
 // ICDE 1997): sort by x and cut into sx slabs of whole tiles; sort each slab
@@ -519,20 +534,12 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
       }
       mol->host_launches += 7;
     } else {
-      double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-      for (int a = 0; a < mol->natom; ++a)
-        for (int d = 0; d < 3; ++d) {
-          lo[d] = std::min(lo[d], mol->atom_xyz[3 * a + d]);
-          hi[d] = std::max(hi[d], mol->atom_xyz[3 * a + d]);
-        }
-      if (mol->natom == 0)
-        for (int d = 0; d < 3; ++d) { lo[d] = -1; hi[d] = 1; }
-      double ext = 0;
-      for (int d = 0; d < 3; ++d) ext = std::max(ext, hi[d] - lo[d] + 24.0);
+      double lo[3], ext = 0;
+      morton_box(mol, lo, &ext);
       uint32_t* k32_in = (uint32_t*)k_in;
       uint32_t* k32_out = (uint32_t*)k_out;
-      morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src.pts, n, lo[0] - 12.0, lo[1] - 12.0,
-                                                                  lo[2] - 12.0, 1024.0 / ext, k32_in, v_in);
+      morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src.pts, n, lo[0], lo[1], lo[2], 1024.0 / ext,
+                                                                  k32_in, v_in);
       CTC_CUDA_TRY(cudaGetLastError());
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k32_in, k32_out, v_in, perm, (int)n, 0,
                                                    kMortonSortBits, st));
