@@ -60,7 +60,7 @@ namespace {
 
 constexpr int kLmax = 8;                 // g x g
 constexpr int kTaylor = 7;               // terms of the Taylor expansion
-constexpr int kRow = kTaylor + 1;         // table row: Taylor coefficients, e^{-T_i}
+constexpr int kRow = 2;                  // table row of class L: F_{L+6}(T_i), e^{-T_i}
 constexpr double kTstep = 0.05;
 constexpr double kTmax = 64.0;           // table range: above every far_T(L <= 8)
 constexpr int kNT = (int)(kTmax / kTstep) + 2;
@@ -85,11 +85,19 @@ struct EspPair {
 };
 struct EspBatch {
   int32_t b0, b1;   // pairs [b0, b1)
-  int32_t h0;       // first Hermite coefficient
-  int32_t f0;       // first far-field coefficient (nfar(L) per pair)
-  int32_t L;
-  int32_t pad[3];
+  int64_t h0;       // first near-field coefficient (nnear(L) per pair)
+  int64_t f0;       // first far-field coefficient (nfar(L) per pair)
+  int32_t L, pad;
 };
+// Near-field polynomials: sum_tuv h_tuv R_tuv = sum_n G_n p_n(X, Y, Z), p_n of
+// the degrees 2n - s for n <= s <= min(2n, L).
+__host__ __device__ constexpr int near_lo(int L, int n) { return 2 * n > L ? 2 * n - L : 0; }
+__host__ __device__ constexpr int nnear(int L) {
+  int c = 0;
+  for (int n = 0; n <= L; ++n)
+    for (int d = near_lo(L, n); d <= n; ++d) c += (d + 1) * (d + 2) / 2;
+  return c;
+}
 // far-field coefficients of a pair besides the constant one, padded to whole
 // 16-byte loads
 __host__ __device__ constexpr int nfar(int L) { return ntuv(L) / 2 * 2; }
@@ -117,12 +125,11 @@ __host__ __device__ constexpr int batch_pairs(int L) {
 struct EspTables {
   double* d_boys = nullptr;
   EspPair* d_pairs = nullptr;
-  double* d_h = nullptr;
+  double* d_h = nullptr;      // near-field polynomials, nnear(L) per pair
   double* d_far = nullptr;    // far-field polynomials, nfar(L) per pair
   EspBatch* d_batches = nullptr;
   double* d_atoms = nullptr;  // x y z Z per atom
   int npairs = 0, nbatch = 0, natom = 0;
-  int Lmax = 0;  // largest class with pairs
   size_t nh = 0;
   // algorithmic FP64 work per point: sum over the kept pairs of
   // 2 n_tuv(L) (contraction) + 2 n_R(L) (R recursion) + 10 (L + 1) (Boys)
@@ -143,11 +150,13 @@ __host__ __device__ constexpr double far_T(int L) { return 38.0 + 3.0 * L; }
 // G_n = R^n_000 = (-2p)^n F_n(T), n = 0..L, at T = p r2.
 //  far field (T >= far_T(L)): the p dependence cancels except in F_0,
 //    G_0 = (sqrt(pi/p)/2) / r,  G_n = -(2n-1) G_{n-1} / r2  -- no exponential;
-//  otherwise: F_L from the 7-term Taylor expansion about the nearest 0.05 step
-//    T_i (class L's table: coefficients F_{L+k}(T_i) / k! in d = T_i - T, then
-//    e^{-T_i}: one 64-byte row), e^{-T} = e^{-T_i} e^d with e^d by its series to
-//    d^7 (|d| <= 0.025: remainder below 4e-18),
-//    F_{n-1} = (2T F_n + e^{-T}) / (2n-1) downwards (stable for every T).
+//  otherwise: from one 16-byte table row at the nearest 0.05 step T_i,
+//    F_{L+6}(T_i) and e^{-T_i}: F_{L+5} .. F_L there by downward recursion, F_L(T)
+//    by the 7-term Taylor expansion in d = T_i - T, e^{-T} = e^{-T_i} e^d with e^d
+//    by its series to d^7 (|d| <= 0.025: remainder below 4e-18), and
+//    F_{n-1} = (2T F_n + e^{-T}) / (2n-1) downwards (stable for every T).  The
+//    lanes' rows lie far apart, so the row's size is what the L1 sees: reading
+//    the seven coefficients (64 bytes in four loads) bound the near kernel.
 template <int L>
 __device__ __forceinline__ void boys_g(double p, double f0c, double r2, const double* __restrict__ tab,
                                        double* G) {
@@ -161,10 +170,17 @@ __device__ __forceinline__ void boys_g(double p, double f0c, double r2, const do
   } else {
     const int i = __double2int_rn(T * (1.0 / kTstep));
     const double d = i * kTstep - T;  // T_i - T
-    const double2* row = reinterpret_cast<const double2*>(tab + ((int64_t)L * kNT + i) * kRow);
-    const double2 c01 = __ldg(row), c23 = __ldg(row + 1), c45 = __ldg(row + 2), c6e = __ldg(row + 3);
-    double F[L + 1];
-    F[L] = fma(fma(fma(fma(fma(fma(c6e.x, d, c45.y), d, c45.x), d, c23.y), d, c23.x), d, c01.y), d, c01.x);
+    const double2 row = __ldg(reinterpret_cast<const double2*>(tab) + ((int64_t)L * kNT + i));
+    double F[L + 1], f[kTaylor];
+    const double Ti2 = 2.0 * (i * kTstep);
+    f[kTaylor - 1] = row.x;
+#pragma unroll
+    for (int k = kTaylor - 1; k > 0; --k)
+      f[k - 1] = fma(Ti2, f[k], row.y) * (1.0 / (double)(2 * (L + k) - 1));
+    double fl = f[kTaylor - 1];
+#pragma unroll
+    for (int k = kTaylor - 2; k >= 0; --k) fl = fma(fl * d, 1.0 / (double)(k + 1), f[k]);
+    F[L] = fl;
     if (L > 0) {
       double q = 1.0 / 5040.0;
       q = fma(q, d, 1.0 / 720.0);
@@ -174,7 +190,7 @@ __device__ __forceinline__ void boys_g(double p, double f0c, double r2, const do
       q = fma(q, d, 0.5);
       q = fma(q, d, 1.0);
       q = fma(q, d, 1.0);
-      const double e = c6e.y * q, T2 = 2.0 * T;
+      const double e = row.y * q, T2 = 2.0 * T;
 #pragma unroll
       for (int n = L; n > 0; --n) F[n - 1] = fma(T2, F[n], e) * (1.0 / (double)(2 * n - 1));
     }
@@ -187,38 +203,40 @@ __device__ __forceinline__ void boys_g(double p, double f0c, double r2, const do
   }
 }
 
-// R^0_{tuv}(p, X, Y, Z) for t+u+v <= L, in place from level L down to 0,
-// from G_n = R^n_000.
+// sum_n G_n p_n(X, Y, Z) of one pair, the p_n in nested Horner form with the
+// coefficients in the order of their use (n ascending; powers of X, then Y, then
+// Z, descending).  Operations for L = 0..4: 1, 5, 15, 34, 66, about half of the
+// R recursion and its dot product with h.
 template <int L>
-__device__ __forceinline__ void hermite_r(double X, double Y, double Z, const double* G, double* R) {
-  R[0] = G[L];
+__device__ __forceinline__ double near_sum(double X, double Y, double Z, const double* G,
+                                           const double* __restrict__ h) {
+  double zp[L + 1];
+  zp[0] = 1.0;
 #pragma unroll
-  for (int n = L - 1; n >= 0; --n) {
-    // level n: totals L-n down to 1 from level n+1, then total 0
+  for (int i = 1; i <= L; ++i) zp[i] = zp[i - 1] * Z;
+  double s = 0.0;
+  int k = 0;
 #pragma unroll
-    for (int s = L - n; s >= 1; --s) {
+  for (int n = 0; n <= L; ++n) {
+    const int dlo = near_lo(L, n);
+    double f = 0.0;
 #pragma unroll
-      for (int t = s; t >= 0; --t) {
+    for (int a = n; a >= 0; --a) {
+      double g = 0.0;
 #pragma unroll
-        for (int u = s - t; u >= 0; --u) {
-          const int v = s - t - u;
-          double r;
-          if (t > 0) {
-            r = X * R[tuv_index(t - 1, u, v)];
-            if (t > 1) r += (t - 1) * R[tuv_index(t - 2, u, v)];
-          } else if (u > 0) {
-            r = Y * R[tuv_index(t, u - 1, v)];
-            if (u > 1) r += (u - 1) * R[tuv_index(t, u - 2, v)];
-          } else {
-            r = Z * R[tuv_index(t, u, v - 1)];
-            if (v > 1) r += (v - 1) * R[tuv_index(t, u, v - 2)];
-          }
-          R[tuv_index(t, u, v)] = r;
-        }
+      for (int b = n - a; b >= 0; --b) {
+        const int lo = dlo > a + b ? dlo - a - b : 0;
+        double t = h[k++];
+#pragma unroll
+        for (int e = n - a - b - 1; e >= lo; --e) t = fma(t, Z, h[k++]);
+        if (lo > 0) t *= zp[lo];
+        g = b == n - a ? t : fma(g, Y, t);
       }
+      f = a == n ? g : fma(f, X, g);
     }
-    R[0] = G[n];
+    s = fma(G[n], f, s);
   }
+  return s;
 }
 
 constexpr int kEspThreads = 128;
@@ -383,8 +401,9 @@ __device__ __forceinline__ void esp_far_pair(const double4 q, const double2* __r
 // Far pairs of block x's points (P per thread) in slice y of the batches of all
 // classes: row y of part.  Rows are summed in a fixed order by
 // esp_finish_kernel, so results do not depend on timing.
-// Bound: FP64 pipe.  100 atoms (1 604 functions, 8e5 pairs), 1e5 surface
-// points: the five class kernels with the R recursion took 287 ms.
+// Bound: FP64 pipe (73% busy).  100 atoms (1 604 functions, 8e5 pairs), 1e5
+// surface points: far 110 ms and near 40 ms; one kernel per class with the R
+// recursion for every pair took 287 ms.
 template <int P>
 __global__ void __launch_bounds__(kEspThreads)
     esp_far_kernel(const EspPair* __restrict__ pairs, const double* __restrict__ far,
@@ -448,10 +467,10 @@ __global__ void __launch_bounds__(kEspThreads)
 
 // Near pairs of the same blocks and slices.  A warp whose points are all far
 // from the pair takes the far-field polynomial, the others the Boys function
-// and the R recursion (far points of such a warp by the asymptotic form).
-// LMAX bounds the classes (the R recursion's registers).
-template <int LMAX, int P>
-__global__ void __launch_bounds__(kEspThreads)
+// and the near-field polynomials (far points of such a warp by the asymptotic
+// form).
+template <int P>
+__global__ void __launch_bounds__(kEspThreads, 7)
     esp_near_kernel(const EspPair* __restrict__ pairs, const double* __restrict__ hbuf,
                     const double* __restrict__ far, const EspBatch* __restrict__ batches, int nb, const double* __restrict__ tab,
                     const double* __restrict__ xyz, int64_t n, double* __restrict__ part) {
@@ -479,41 +498,34 @@ __global__ void __launch_bounds__(kEspThreads)
     __syncthreads();
     const int nn = esp_select<false>(pairs + bt.b0, bt.b1 - bt.b0, ctr, rad, s_list, s_cnt);
     // the near pairs in groups that fit the shared arrays
-    const int NT = ntuv(bt.L), cap = min(kBatchPairs, kBatchH / NT) / 4;
+    const int NT = nnear(bt.L), cap = min(kBatchPairs, kBatchH / NT) / 4;  // (coefficients: 1024)
     for (int g0 = 0; g0 < nn; g0 += cap) {
       const int ng = min(cap, nn - g0);
       __syncthreads();
       for (int i = threadIdx.x; i < ng; i += kEspThreads) sp[i] = pairs[bt.b0 + s_list[g0 + i]];
       for (int i = threadIdx.x; i < ng * NT; i += kEspThreads)
-        sh[i] = hbuf[bt.h0 + (int64_t)s_list[g0 + i / NT] * NT + i % NT];
+        sh[i] = hbuf[bt.h0 + s_list[g0 + i / NT] * NT + i % NT];
       const int NF = nfar(bt.L);
       for (int i = threadIdx.x; i < ng * NF; i += kEspThreads)
-        sf[i] = far[bt.f0 + (int64_t)s_list[g0 + i / NF] * NF + i % NF];
+        sf[i] = far[bt.f0 + s_list[g0 + i / NF] * NF + i % NF];
       __syncthreads();
       auto run = [&](auto lc) {
         constexpr int L = decltype(lc)::value;
-        if constexpr (L <= LMAX) {
-          for (int k = 0; k < ng; ++k) {
-            const EspPair q = sp[k];
-            const double* h = sh + k * ntuv(L);
+        for (int k = 0; k < ng; ++k) {
+          const EspPair q = sp[k];
 #pragma unroll
-            for (int p = 0; p < P; ++p) {
-              const double X = q.Px - c[p][0], Y = q.Py - c[p][1], Z = q.Pz - c[p][2];
-              const double r2 = X * X + Y * Y + Z * Z;
-              if (__all_sync(0xffffffffu, q.p * r2 >= far_T(L))) {
-                esp_far_pair<L, 1>(make_double4(q.Px, q.Py, q.Pz, q.c0),
-                                   reinterpret_cast<const double2*>(sf) + k * (nfar(L) / 2), c + p, acc + p);
-                continue;
-              }
-              double G[L + 1];
-              boys_g<L>(q.p, q.f0c, r2, tab, G);
-              double R[ntuv(L)];
-              hermite_r<L>(X, Y, Z, G, R);
-              double s = 0.0;
-#pragma unroll
-              for (int j = 0; j < ntuv(L); ++j) s += h[j] * R[j];
-              acc[p] += s;
+          for (int p = 0; p < P; ++p) {
+            const double X = q.Px - c[p][0], Y = q.Py - c[p][1], Z = q.Pz - c[p][2];
+            const double r2 = X * X + Y * Y + Z * Z;
+            // (beyond 1e30 bohr the powers of X overflow: far form also in a mixed warp)
+            if (__all_sync(0xffffffffu, q.p * r2 >= far_T(L)) || r2 > 1e60) {
+              esp_far_pair<L, 1>(make_double4(q.Px, q.Py, q.Pz, q.c0),
+                                 reinterpret_cast<const double2*>(sf) + k * (nfar(L) / 2), c + p, acc + p);
+              continue;
             }
+            double G[L + 1];
+            boys_g<L>(q.p, q.f0c, r2, tab, G);
+            acc[p] += near_sum<L>(X, Y, Z, G, sh + k * nnear(L));
           }
         }
       };
@@ -603,6 +615,33 @@ struct PairOut {
   EspPair pr;
   std::vector<double> h;
 };
+
+// Near-field polynomials of a pair, in near_sum's order, from
+//   R_tuv = sum_ijk a_ti a_uj a_vk X^(t-2i) Y^(u-2j) Z^(v-2k) G_(t+u+v-i-j-k),
+// a_ti = t! / (2^i i! (t - 2i)!), the solved recursion R^n_{t+1} = X R^(n+1)_t +
+// t R^(n+1)_{t-1}.
+void near_coefficients(int L, const double* h, double* out) {
+  auto term = [](int t, int i) {
+    double v = 1.0;
+    for (int k = 0; k < 2 * i; ++k) v *= t - k;
+    for (int k = 1; k <= i; ++k) v /= 2.0 * k;
+    return v;
+  };
+  int k = 0;
+  for (int n = 0; n <= L; ++n)
+    for (int a = n; a >= 0; --a)
+      for (int b = n - a; b >= 0; --b)
+        for (int c = n - a - b; c >= (near_lo(L, n) > a + b ? near_lo(L, n) - a - b : 0); --c) {
+          const int m = n - (a + b + c);  // i + j + k
+          double s = 0.0;
+          for (int i = 0; i <= m; ++i)
+            for (int j = 0; i + j <= m; ++j) {
+              const int t = a + 2 * i, u = b + 2 * j, v = c + 2 * (m - i - j);
+              s += h[tuv_index(t, u, v)] * term(t, i) * term(u, j) * term(v, m - i - j);
+            }
+          out[k++] = s;
+        }
+}
 
 // Far-field polynomial of a pair.  d_x^t d_y^u d_z^v (1/r) = Q_tuv r^(-2l-1),
 // l = t + u + v, with Q_000 = 1 and Q_{t+1,u,v} = r^2 d_x Q - (2l+1) x Q (the
@@ -807,27 +846,28 @@ static int build_esp(ctc_molecule* mol) {
   std::vector<EspPair> pairs;
   std::vector<double> hv, fv;
   std::vector<EspBatch> batches;
-  int Lmax = 0;
   static const FarTerms far_terms;
+  size_t nh = 0;  // Hermite coefficients
   for (int L = 0; L <= kLmax; ++L) {
     const int per = batch_pairs(L);
     int in_batch = 0;
     for (auto& o : outs)
       for (auto& po : o) {
         if (po.L != L) continue;
-        Lmax = L;
         if (in_batch == 0)
-          batches.push_back({(int32_t)pairs.size(), (int32_t)pairs.size(), (int32_t)hv.size(), (int32_t)fv.size(), L, {0, 0, 0}});
+          batches.push_back({(int32_t)pairs.size(), (int32_t)pairs.size(), (int64_t)hv.size(), (int64_t)fv.size(), L, 0});
         double fc[ntuv(kLmax) + 1];
         po.pr.c0 = far_terms.of(L, po.h.data(), po.pr.f0c, fc);
         fv.insert(fv.end(), fc, fc + nfar(L));
         pairs.push_back(po.pr);
-        hv.insert(hv.end(), po.h.begin(), po.h.end());
+        hv.resize(hv.size() + nnear(L));
+        near_coefficients(L, po.h.data(), hv.data() + hv.size() - nnear(L));
+        nh += ntuv(L);
         batches.back().b1 = (int32_t)pairs.size();
         if (++in_batch == per) in_batch = 0;
       }
   }
-  if (hv.size() > (size_t)INT32_MAX) return fail(CTC_ERR_UNSUPPORTED, "ESP: too many pair coefficients");
+  if (nh > (size_t)INT32_MAX) return fail(CTC_ERR_UNSUPPORTED, "ESP: too many pair coefficients");
   // Boys table
   std::vector<double> tab((size_t)(kLmax + 1) * kNT * kRow);
   for (int i = 0; i < kNT; ++i) {
@@ -835,12 +875,8 @@ static int build_esp(ctc_molecule* mol) {
     for (int m = 0; m < kLmax + kTaylor; ++m) F[m] = boys_series(m, i * kTstep);
     for (int L = 0; L <= kLmax; ++L) {
       double* row = &tab[((size_t)L * kNT + i) * kRow];
-      double fact = 1.0;
-      for (int k = 0; k < kTaylor; ++k) {
-        row[k] = F[L + k] / fact;
-        fact *= k + 1;
-      }
-      row[kTaylor] = std::exp(-i * kTstep);
+      row[0] = F[L + kTaylor - 1];
+      row[1] = std::exp(-i * kTstep);
     }
   }
   std::vector<double> atoms(4 * (size_t)std::max(mol->natom, 1));
@@ -860,11 +896,10 @@ static int build_esp(ctc_molecule* mol) {
     e->mean_L += (double)np * bt.L;
   }
   if (!pairs.empty()) e->mean_L /= (double)pairs.size();
-  e->Lmax = Lmax;
   e->npairs = (int)pairs.size();
   e->nbatch = (int)batches.size();
   e->natom = mol->natom;
-  e->nh = hv.size();
+  e->nh = nh;
   auto up = [&](void** dst, const void* src, size_t bytes) -> int {
     if (bytes == 0) bytes = 8;
     CTC_CUDA_TRY(cudaMalloc(dst, bytes));
@@ -917,8 +952,8 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
     const double* pts = d_points + 3 * p0;
     // two points per thread share a pair's coefficients; one when the points
     // would fill less than a block per SM (the pairs are then cut into more
-    // slices) or the R recursion of classes above 4 needs all registers
-    const int P = e->Lmax <= 4 && m >= (int64_t)2 * kEspThreads * nsm ? 2 : 1;
+    // slices)
+    const int P = m >= (int64_t)2 * kEspThreads * nsm ? 2 : 1;
     const int64_t gx = (m + P * kEspThreads - 1) / (P * kEspThreads);
     // slices of the batches: about 32 blocks per SM, at least a batch each
     const int64_t want = (32 * (int64_t)nsm + gx - 1) / gx;
@@ -956,16 +991,8 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
       if (P == 2) esp_far_kernel<2><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_far, e->d_batches, e->nbatch, xyz, m, part);
       else esp_far_kernel<1><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_far, e->d_batches, e->nbatch, xyz, m, part);
       CTC_CUDA_TRY(cudaGetLastError());
-#define CTC_ESP_NEAR(LM, PP)                                                                                       \
-  esp_near_kernel<LM, PP><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch,      \
-                                                       e->d_boys, xyz, m, near)
-      if (e->Lmax > 6) CTC_ESP_NEAR(8, 1);
-      else if (e->Lmax > 4) CTC_ESP_NEAR(6, 1);
-      else if (e->Lmax > 2 && P == 2) CTC_ESP_NEAR(4, 2);
-      else if (e->Lmax > 2) CTC_ESP_NEAR(4, 1);
-      else if (P == 2) CTC_ESP_NEAR(2, 2);
-      else CTC_ESP_NEAR(2, 1);
-#undef CTC_ESP_NEAR
+      if (P == 2) esp_near_kernel<2><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
+      else esp_near_kernel<1><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
       CTC_CUDA_TRY(cudaGetLastError());
     }
     esp_finish_kernel<<<g, 256, 0, st>>>(part, 2 * S, e->d_atoms, e->natom, xyz, perm, m, d_out + p0);
