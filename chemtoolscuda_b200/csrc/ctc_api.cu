@@ -175,9 +175,7 @@ int ctc_eval_ao(ctc_molecule* mol, const double* d_points, int64_t n, int32_t de
   if (!mol || !d_out || (n > 0 && !d_points)) return fail(CTC_ERR_INVALID, "ctc_eval_ao: null argument");
   if (deriv < 0 || deriv > 2) return fail(CTC_ERR_INVALID, "ctc_eval_ao: deriv must be 0, 1 or 2");
   if (n <= 0) return n < 0 ? fail(CTC_ERR_INVALID, "ctc_eval_ao: negative point count") : CTC_OK;
-  PointSrc src{};
-  src.pts = d_points;
-  return launch_ao_public(mol, src, n, deriv, d_out, (cudaStream_t)stream);
+  return launch_ao_public(mol, d_points, n, deriv, d_out, (cudaStream_t)stream);
 }
 
 int ctc_eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out, void* stream) {

@@ -420,9 +420,24 @@ int ctc_molecule_create(const ctc_basis* b, int32_t natom, const double* atom_xy
   m->seg_order.resize(m->nseg);
   for (int i = 0; i < m->nseg; ++i) m->seg_order[i] = i;
   std::stable_sort(m->seg_order.begin(), m->seg_order.end(), [&](int x, int y) {
-    if (m->segs[x].type != m->segs[y].type) return m->segs[x].type < m->segs[y].type;
-    return m->segs[x].nprim < m->segs[y].nprim;
+    return m->segs[x].orig_ao0 < m->segs[y].orig_ao0;
   });
+  // runs of whole segments with at most 64 or 32 AOs (the widest segment has 15)
+  std::vector<int2> chunks[2];
+  for (int k = 0; k < 2; ++k) {
+    int first = 0, count = 0;
+    for (int i = 0; i < m->nseg; ++i) {
+      const int nc = ncomp_of_type(m->segs[m->seg_order[i]].type);
+      if (count + nc > (k ? 32 : 64)) {
+        chunks[k].push_back(make_int2(first, i));
+        first = i;
+        count = 0;
+      }
+      count += nc;
+    }
+    chunks[k].push_back(make_int2(first, m->nseg));
+    m->n_aochunk[k] = (int)chunks[k].size();
+  }
   m->D.resize((size_t)ao * ao);
   for (int i = 0; i < ao; ++i) {
     const double* src = D + (size_t)m->ao_perm[i] * ao;
@@ -450,6 +465,8 @@ int ctc_molecule_create(const ctc_basis* b, int32_t natom, const double* atom_xy
   ALLOC_COPY(m->d_alpha, m->alpha.data(), m->alpha.size());
   ALLOC_COPY(m->d_coef, m->coef.data(), m->coef.size());
   ALLOC_COPY(m->d_order, m->seg_order.data(), m->seg_order.size());
+  ALLOC_COPY(m->d_aochunk[0], chunks[0].data(), chunks[0].size());
+  ALLOC_COPY(m->d_aochunk[1], chunks[1].data(), chunks[1].size());
   ALLOC_COPY(m->d_ao_atom, m->ao_atom.data(), m->ao_atom.size());
   ALLOC_COPY(m->d_D, Dpad.data(), MM);
   ALLOC_COPY(m->d_ao_iperm, iperm.data(), iperm.size());
@@ -478,6 +495,8 @@ int ctc_molecule_destroy(ctc_molecule* m) {
   cudaFree(m->d_alpha);
   cudaFree(m->d_coef);
   cudaFree(m->d_order);
+  cudaFree(m->d_aochunk[0]);
+  cudaFree(m->d_aochunk[1]);
   cudaFree(m->d_ao_atom);
   cudaFree(m->d_D);
   cudaFree(m->d_sym);

@@ -142,7 +142,7 @@ struct ctc_molecule {
   int natom = 0, M = 0, Mpad = 0, nseg = 0;
   std::vector<ctc::DevSeg> segs;             // host copy
   std::vector<double> alpha, coef;           // host copies (coef includes N_l(alpha))
-  std::vector<int32_t> seg_order;            // segments sorted by type, nprim
+  std::vector<int32_t> seg_order;            // segments in the caller's AO order
   std::vector<double> atom_xyz, charges;
   std::vector<double> D;                     // host copy, M x M
   std::vector<int32_t> ao_atom;              // AO -> atom (internal order)
@@ -154,7 +154,9 @@ struct ctc_molecule {
   ctc::DevSeg* d_segs = nullptr;
   double* d_alpha = nullptr;
   double* d_coef = nullptr;
-  int32_t* d_order = nullptr;
+  int32_t* d_order = nullptr;                // seg_order
+  int2* d_aochunk[2] = {nullptr, nullptr};   // runs of seg_order with at most 64 (0) or 32 (1) AOs
+  int n_aochunk[2] = {0, 0};
   int32_t* d_ao_atom = nullptr;
   double* d_D = nullptr;                     // Mpad x Mpad, zero padded
   int32_t* d_sym = nullptr;                  // 1: D is symmetric (set_symmetry_flag)
@@ -206,8 +208,8 @@ int launch_ao_tiles_weighted(const ctc_molecule* mol, const TileBatch& tb, const
 int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int deriv, int nqa,
                            int8_t* planes, int32_t* eexp, const int32_t* order, cudaStream_t st);
 // AO output in (nq, n, M) layout for ctc_eval_ao.
-int launch_ao_public(const ctc_molecule* mol, const PointSrc& src, int64_t n, int deriv,
-                     double* out, cudaStream_t st);
+int launch_ao_public(const ctc_molecule* mol, const double* pts, int64_t n, int deriv, double* out,
+                     cudaStream_t st);
 
 // ---- local descriptors (ctc_local.cu) ----
 struct LocalPlan {
