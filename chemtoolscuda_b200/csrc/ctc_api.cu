@@ -276,9 +276,12 @@ int ctc_eval_local_host(ctc_molecule* mol, const double* h_points, int64_t n, in
   }
   drain(b);
   drain(b ^ 1);
-  // a device-side failure of the tensor-core kernels of this call
-  if (rc == CTC_OK) rc = check_status(mol, cs, "ctc_eval_local_host");
-  // leave nothing of this call in flight (also after an error)
+  if (rc == CTC_OK) {
+    // the last slab's results have arrived, and with them every copy and
+    // kernel of this call: the status copy behind its kernels has landed too
+    return landed_status(mol, cs, "ctc_eval_local_host");
+  }
+  // leave nothing of this call in flight after an error either
   cudaStreamSynchronize(cs);
   cudaStreamSynchronize(h2d);
   cudaStreamSynchronize(d2h);
@@ -289,16 +292,25 @@ int ctc_eval_esp_host(ctc_molecule* mol, const double* h_points, int64_t n, doub
   if (!mol || !h_out || (n > 0 && !h_points)) return fail(CTC_ERR_INVALID, "ctc_eval_esp_host: null argument");
   if (n < 0) return fail(CTC_ERR_INVALID, "ctc_eval_esp_host: negative point count");
   if (n == 0) return CTC_OK;
+  // the device copies of points and results stay with the molecule (up to 32
+  // MiB; larger calls give theirs back)
+  const size_t bytes = sizeof(double) * 4 * (size_t)n;
+  const bool keep = bytes <= (size_t)32 << 20;
   double* d = nullptr;
-  if (cudaMalloc((void**)&d, sizeof(double) * 4 * (size_t)n) != cudaSuccess)
+  if (keep) {
+    if (int rc = mol->ws_io.ensure(bytes, 0); rc != CTC_OK) return rc;
+    d = (double*)mol->ws_io.p;
+  } else if (cudaMalloc((void**)&d, bytes) != cudaSuccess) {
+    cudaGetLastError();
     return fail(CTC_ERR_NOMEM, "ctc_eval_esp_host: device allocation failed");
+  }
   int rc = CTC_OK;
   if (cudaMemcpy(d, h_points, sizeof(double) * 3 * n, cudaMemcpyHostToDevice) != cudaSuccess)
     rc = fail(CTC_ERR_CUDA, "ctc_eval_esp_host: H2D copy failed");
   if (rc == CTC_OK) rc = eval_esp(mol, d, n, d + 3 * n, 0);
   if (rc == CTC_OK && cudaMemcpy(h_out, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = fail(CTC_ERR_CUDA, "ctc_eval_esp_host: D2H copy failed");
-  cudaFree(d);
+  if (!keep) cudaFree(d);
   return rc;
 }
 

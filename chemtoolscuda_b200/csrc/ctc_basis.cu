@@ -237,6 +237,12 @@ int check_status(ctc_molecule* mol, cudaStream_t st, const char* what) {
   return report_status(mol, st, what);
 }
 
+int landed_status(ctc_molecule* mol, cudaStream_t st, const char* what) {
+  if (mol->status_pending) CTC_CUDA_TRY(cudaEventSynchronize(mol->status_ev));
+  mol->status_pending = false;
+  return report_status(mol, st, what);
+}
+
 // Radius beyond which |AO|, |grad AO| and |hess AO| of a segment stay below
 // eps for every component: a conservative bound using the largest polynomial
 // coefficient of the segment's type.
@@ -516,6 +522,7 @@ int ctc_molecule_destroy(ctc_molecule* m) {
   m->ws_cap.release();
   m->ws_esp.release();
   m->ws_adj.release();
+  m->ws_io.release();
   if (m->hostpipe) {
     m->hostpipe->release();
     delete m->hostpipe;

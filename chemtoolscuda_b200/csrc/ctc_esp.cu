@@ -21,13 +21,14 @@
 // H a polynomial of degree L with n_tuv(L) coefficients formed at set-up: one
 // reciprocal square root and one multiply-add per coefficient, instead of the R
 // recursion and a dot product (FP64 operations per pair and point for L = 0..4:
-// 12, 19, 25, 35, 50).  esp_far_kernel sums these pairs, all classes in one
+// 12, 17, 25, 35, 50).  esp_far_kernel sums these pairs, all classes in one
 // launch, two points per thread.  Points are sorted along a Morton curve, so a
 // block's points lie close together and few pairs are near one of them and far
 // from the others.
 //
-// Near pairs of a block (a few per cent) go to esp_near_kernel: Boys function,
-// R recursion and the dot product with h, per point.
+// Near pairs of a block (a few per cent) go to esp_near_kernel: Boys function
+// and sum_n G_n p_n(P - C), G_n = (-2p)^n F_n, with polynomials p_n formed at
+// set-up (half the operations of the R recursion and its dot product with h).
 //
 // Boys function F_n(T) (FP64): beyond a per-L threshold (T >= 38 + 3L, where
 // the neglected e^{-T} terms are below 2e-17 relative) the asymptotic forms
@@ -616,50 +617,50 @@ struct PairOut {
   std::vector<double> h;
 };
 
-// Near-field polynomials of a pair, in near_sum's order, from
-//   R_tuv = sum_ijk a_ti a_uj a_vk X^(t-2i) Y^(u-2j) Z^(v-2k) G_(t+u+v-i-j-k),
-// a_ti = t! / (2^i i! (t - 2i)!), the solved recursion R^n_{t+1} = X R^(n+1)_t +
-// t R^(n+1)_{t-1}.
-void near_coefficients(int L, const double* h, double* out) {
-  auto term = [](int t, int i) {
-    double v = 1.0;
-    for (int k = 0; k < 2 * i; ++k) v *= t - k;
-    for (int k = 1; k <= i; ++k) v /= 2.0 * k;
-    return v;
-  };
-  int k = 0;
-  for (int n = 0; n <= L; ++n)
-    for (int a = n; a >= 0; --a)
-      for (int b = n - a; b >= 0; --b)
-        for (int c = n - a - b; c >= (near_lo(L, n) > a + b ? near_lo(L, n) - a - b : 0); --c) {
-          const int m = n - (a + b + c);  // i + j + k
-          double s = 0.0;
-          for (int i = 0; i <= m; ++i)
-            for (int j = 0; i + j <= m; ++j) {
-              const int t = a + 2 * i, u = b + 2 * j, v = c + 2 * (m - i - j);
-              s += h[tuv_index(t, u, v)] * term(t, i) * term(u, j) * term(v, m - i - j);
+// Coefficients of a pair's polynomials as linear maps of its Hermite
+// coefficients h, one sparse list of (output, input, factor) per class.
+struct MapTerm {
+  int16_t out, in;
+  double f;
+};
+struct EspMaps {
+  std::vector<MapTerm> near[kLmax + 1];  // outputs in near_sum's order
+  std::vector<MapTerm> far[kLmax + 1];   // outputs in esp_far_pair's order, the constant one last
+  EspMaps() {
+    // Near field: R_tuv = sum_ijk a_ti a_uj a_vk X^(t-2i) Y^(u-2j) Z^(v-2k) G_(t+u+v-i-j-k),
+    // a_ti = t! / (2^i i! (t - 2i)!), the solved recursion R^n_{t+1} = X R^(n+1)_t + t R^(n+1)_{t-1}.
+    auto fac = [](int t, int i) {
+      double v = 1.0;
+      for (int k = 0; k < 2 * i; ++k) v *= t - k;
+      for (int k = 1; k <= i; ++k) v /= 2.0 * k;
+      return v;
+    };
+    for (int L = 0; L <= kLmax; ++L) {
+      int k = 0;
+      for (int n = 0; n <= L; ++n)
+        for (int a = n; a >= 0; --a)
+          for (int b = n - a; b >= 0; --b)
+            for (int c = n - a - b; c >= std::max(0, near_lo(L, n) - a - b); --c, ++k) {
+              const int m = n - (a + b + c);  // i + j + k
+              for (int i = 0; i <= m; ++i)
+                for (int j = 0; i + j <= m; ++j) {
+                  const int t = a + 2 * i, u = b + 2 * j, v = c + 2 * (m - i - j);
+                  near[L].push_back({(int16_t)k, (int16_t)tuv_index(t, u, v), fac(t, i) * fac(u, j) * fac(v, m - i - j)});
+                }
             }
-          out[k++] = s;
-        }
-}
-
-// Far-field polynomial of a pair.  d_x^t d_y^u d_z^v (1/r) = Q_tuv r^(-2l-1),
-// l = t + u + v, with Q_000 = 1 and Q_{t+1,u,v} = r^2 d_x Q - (2l+1) x Q (the
-// same for y, z): homogeneous of degree l with integer coefficients.  With
-// (x, y, z) scaled by 1/r^2, sum_tuv h_tuv Q_tuv r^(-2l-1) is 1/r times one
-// polynomial of degree L.
-struct FarTerms {
-  // q[tuv]: coefficients of Q_tuv by tuv_index of the monomial's exponents,
-  // from the first monomial of its degree
-  std::vector<std::vector<double>> q;
-  FarTerms() : q(ntuv(kLmax)) {
+    }
+    // Far field: d_x^t d_y^u d_z^v (1/r) = Q_tuv r^(-2l-1), l = t + u + v, with
+    // Q_000 = 1 and Q_{t+1,u,v} = r^2 d_x Q - (2l+1) x Q (the same for y, z):
+    // homogeneous of degree l with integer coefficients.  With (x, y, z) scaled
+    // by 1/r^2, sum_tuv h_tuv Q_tuv r^(-2l-1) is 1/r times one polynomial.
+    // q[tuv]: coefficients by tuv_index of the monomial, from its degree's first
+    std::vector<std::vector<double>> q(ntuv(kLmax));
     q[0] = {1.0};
     for (int s = 1; s <= kLmax; ++s)
       for (int t = s; t >= 0; --t)
         for (int u = s - t; u >= 0; --u) {
-          const int e[3] = {t, u, s - t - u};
-          const int ax = e[0] ? 0 : (e[1] ? 1 : 2);
-          int low[3] = {e[0], e[1], e[2]};
+          int low[3] = {t, u, s - t - u};
+          const int ax = low[0] ? 0 : (low[1] ? 1 : 2);
           --low[ax];
           const int l = s - 1, base_l = ntuv(l - 1), base_s = ntuv(s - 1);
           const std::vector<double>& ql = q[tuv_index(low[0], low[1], low[2])];
@@ -679,29 +680,39 @@ struct FarTerms {
             }
           q[tuv_index(t, u, s - t - u)] = std::move(r);
         }
-  }
-  // coefficients in Horner order, times f0c; returns the constant one
-  double of(int L, const double* h, double f0c, double* out) const {
-    double poly[ntuv(kLmax)] = {};
-    for (int i = 0, s = 0; i < ntuv(L); ++i) {
-      if (i == ntuv(s)) ++s;
-      if (h[i] == 0.0) continue;
-      const int base = ntuv(s - 1);
-      for (size_t m = 0; m < q[i].size(); ++m) poly[base + m] += h[i] * q[i][m];
+    for (int L = 0; L <= kLmax; ++L) {
+      int k = 0;
+      for (int a = L; a >= 0; --a)
+        for (int b = L - a; b >= 0; --b)
+          for (int c = L - a - b; c >= 0; --c, ++k) {
+            const int s = a + b + c, base = ntuv(s - 1), mono = tuv_index(a, b, c) - base;
+            for (int i = base; i < ntuv(s); ++i)
+              if (q[i][mono] != 0.0) far[L].push_back({(int16_t)k, (int16_t)i, q[i][mono]});
+          }
     }
-    int k = 0;
-    for (int a = L; a >= 0; --a)
-      for (int b = L - a; b >= 0; --b)
-        for (int c = L - a - b; c >= 0; --c)
-          if (a || b || c) out[k++] = f0c * poly[tuv_index(a, b, c)];
-    while (k < nfar(L)) out[k++] = 0.0;
-    return f0c * poly[0];
   }
 };
 
 // Upper bound of |R^0_tuv(p, X)| over all points for t + u + v = s, used to
 // bound a pair's contribution: (2p)^(s/2) times a generous constant in s.
 inline double r_bound(double p, int s) { return std::pow(2.0 * p + 1.0, 0.5 * s) * std::pow(3.0, s); }
+
+// The Boys table of every class (it depends on nothing else: formed once).
+const std::vector<double>& boys_table() {
+  static const std::vector<double> table = [] {
+    std::vector<double> tab((size_t)(kLmax + 1) * kNT * kRow);
+    for (int i = 0; i < kNT; ++i) {
+      const double e = std::exp(-i * kTstep);
+      for (int L = 0; L <= kLmax; ++L) {
+        double* row = &tab[((size_t)L * kNT + i) * kRow];
+        row[0] = boys_series(L + kTaylor - 1, i * kTstep);
+        row[1] = e;
+      }
+    }
+    return tab;
+  }();
+  return table;
+}
 
 }  // namespace
 
@@ -844,41 +855,55 @@ static int build_esp(ctc_molecule* mol) {
   }
   // gather, sorted by L, into batches of equal L
   std::vector<EspPair> pairs;
-  std::vector<double> hv, fv;
+  std::vector<double> hh;  // Hermite coefficients, ntuv(L) per pair
   std::vector<EspBatch> batches;
-  static const FarTerms far_terms;
-  size_t nh = 0;  // Hermite coefficients
+  size_t nnear_all = 0, nfar_all = 0;
+  std::vector<size_t> batch_hh;
   for (int L = 0; L <= kLmax; ++L) {
     const int per = batch_pairs(L);
     int in_batch = 0;
     for (auto& o : outs)
       for (auto& po : o) {
         if (po.L != L) continue;
-        if (in_batch == 0)
-          batches.push_back({(int32_t)pairs.size(), (int32_t)pairs.size(), (int64_t)hv.size(), (int64_t)fv.size(), L, 0});
-        double fc[ntuv(kLmax) + 1];
-        po.pr.c0 = far_terms.of(L, po.h.data(), po.pr.f0c, fc);
-        fv.insert(fv.end(), fc, fc + nfar(L));
+        if (in_batch == 0) {
+          batches.push_back({(int32_t)pairs.size(), (int32_t)pairs.size(), (int64_t)nnear_all, (int64_t)nfar_all, L, 0});
+          batch_hh.push_back(hh.size());
+        }
         pairs.push_back(po.pr);
-        hv.resize(hv.size() + nnear(L));
-        near_coefficients(L, po.h.data(), hv.data() + hv.size() - nnear(L));
-        nh += ntuv(L);
+        hh.insert(hh.end(), po.h.begin(), po.h.end());
+        nnear_all += nnear(L);
+        nfar_all += nfar(L);
         batches.back().b1 = (int32_t)pairs.size();
         if (++in_batch == per) in_batch = 0;
       }
   }
-  if (nh > (size_t)INT32_MAX) return fail(CTC_ERR_UNSUPPORTED, "ESP: too many pair coefficients");
-  // Boys table
-  std::vector<double> tab((size_t)(kLmax + 1) * kNT * kRow);
-  for (int i = 0; i < kNT; ++i) {
-    double F[kLmax + kTaylor];
-    for (int m = 0; m < kLmax + kTaylor; ++m) F[m] = boys_series(m, i * kTstep);
-    for (int L = 0; L <= kLmax; ++L) {
-      double* row = &tab[((size_t)L * kNT + i) * kRow];
-      row[0] = F[L + kTaylor - 1];
-      row[1] = std::exp(-i * kTstep);
-    }
+  if (hh.size() > (size_t)INT32_MAX) return fail(CTC_ERR_UNSUPPORTED, "ESP: too many pair coefficients");
+  // near- and far-field polynomials, batches shared out over the host threads
+  static const EspMaps maps;
+  std::vector<double> hv(nnear_all, 0.0), fv(nfar_all, 0.0);
+  {
+    auto form = [&](size_t first, size_t step) {
+      for (size_t b = first; b < batches.size(); b += step) {
+        const EspBatch& bt = batches[b];
+        const int L = bt.L, last = ntuv(L) - 1;
+        for (int i = bt.b0; i < bt.b1; ++i) {
+          const size_t k = i - bt.b0;
+          const double* h = &hh[batch_hh[b] + k * ntuv(L)];
+          double* nv = hv.data() + bt.h0 + k * nnear(L);
+          double* fp = fv.data() + bt.f0 + k * nfar(L);
+          const double f0c = pairs[i].f0c;
+          for (const MapTerm& t : maps.near[L]) nv[t.out] += t.f * h[t.in];
+          for (const MapTerm& t : maps.far[L]) (t.out == last ? pairs[i].c0 : fp[t.out]) += f0c * t.f * h[t.in];
+        }
+      }
+    };
+    const unsigned nt = (unsigned)std::min<size_t>(nthr, batches.size() / 8 + 1);
+    std::vector<std::thread> tf;
+    for (unsigned t = 1; t < nt; ++t) tf.emplace_back(form, t, nt);
+    form(0, nt);
+    for (auto& t : tf) t.join();
   }
+  const std::vector<double>& tab = boys_table();
   std::vector<double> atoms(4 * (size_t)std::max(mol->natom, 1));
   for (int a = 0; a < mol->natom; ++a) {
     atoms[4 * a] = mol->atom_xyz[3 * a];
@@ -899,7 +924,7 @@ static int build_esp(ctc_molecule* mol) {
   e->npairs = (int)pairs.size();
   e->nbatch = (int)batches.size();
   e->natom = mol->natom;
-  e->nh = nh;
+  e->nh = hh.size();
   auto up = [&](void** dst, const void* src, size_t bytes) -> int {
     if (bytes == 0) bytes = 8;
     CTC_CUDA_TRY(cudaMalloc(dst, bytes));

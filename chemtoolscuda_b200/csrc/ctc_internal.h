@@ -185,7 +185,7 @@ struct ctc_molecule {
   bool prof = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_ev[2];
   // scratch
-  ctc::Scratch ws_ao, ws_sl, ws_part, ws_misc, ws_cap, ws_esp, ws_adj;
+  ctc::Scratch ws_ao, ws_sl, ws_part, ws_misc, ws_cap, ws_esp, ws_adj, ws_io;
   ctc::EspTables* esp = nullptr;
   bool esp_valid = false;
   ctc::HostPipe* hostpipe = nullptr;
@@ -261,6 +261,9 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
 int post_status(ctc_molecule* mol, cudaStream_t st);
 int poll_status(ctc_molecule* mol, cudaStream_t st);
 int check_status(ctc_molecule* mol, cudaStream_t st, const char* what);
+// reports a copy of the word that the caller knows to have landed (its event
+// is waited for; the stream and the device word are not read)
+int landed_status(ctc_molecule* mol, cudaStream_t st, const char* what);
 
 // Records a start/stop event pair around a launch when profiling is on.
 struct ProfScope {

@@ -562,16 +562,28 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   // overrides), at least one full wave of CTAs on 148 SMs.  Larger chunks
   // amortise the per-chunk launches and tails: on the 215^3 benchmark cube
   // 6 GiB gave 20.95 M points/s, 12 GiB 21.46 M, 24 GiB 21.60 M.
-  size_t budget = (size_t)12 << 30;
-  {
+  // The driver is asked for the free memory only when the answer can matter
+  // (the question takes 0.1 to 6 ms on a shared host, as long as a whole call
+  // of 1e5 points): not for calls whose blocks fit what the molecule already
+  // holds or 64 MiB, nor once it holds all that the limit allows.
+  constexpr size_t kMostAo = (size_t)12 << 30, kSmallAo = (size_t)64 << 20;
+  const size_t held = mol->ws_ao.bytes, tile_most = sizeof(double) * (size_t)nq * TP * mol->Mpad;
+  size_t budget = kMostAo;
+  bool asked = false;
+  auto ask = [&]() {
     size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::min(budget, free_b / 4);
+    asked = true;
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) budget = std::max(held, std::min(kMostAo, free_b / 4));
     else cudaGetLastError();  // clear the error; keep the default
-  }
+  };
   if (const char* env = std::getenv("CTC_CHUNK_BYTES")) {
     const long long v = std::atoll(env);
-    if (v > 0) budget = (size_t)v;
+    if (v > 0) {
+      budget = (size_t)v;
+      asked = true;
+    }
   }
+  if (!asked && tile_most * (size_t)ntiles > std::max(held, kSmallAo) && held + tile_most < kMostAo) ask();
   // Capacity of a tile's compact AO set: Mpad always suffices.  When a chunk
   // sized for Mpad columns would hold fewer than four waves of tiles (large
   // bases: the 1 000-atom molecule keeps ~350 of 16 128 functions per tile), a
@@ -602,9 +614,14 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     Kcap = std::min(mol->Mpad, std::max(kKtAlign, (int)mol->h_status[1]));
   }
   const size_t ao_per_tile = sizeof(double) * (size_t)nq * TP * Kcap;
-  int64_t C = std::max<int64_t>(148, (int64_t)(budget / ao_per_tile));
-  C = std::min<int64_t>(C, ntiles);
-  if ((rc = mol->ws_ao.ensure(ao_per_tile * C, st)) != CTC_OK) return rc;
+  int64_t C = 0;
+  for (;;) {
+    C = std::min<int64_t>(std::max<int64_t>(148, (int64_t)(budget / ao_per_tile)), ntiles);
+    rc = mol->ws_ao.ensure(ao_per_tile * C, st);
+    if (rc != CTC_ERR_NOMEM || asked) break;
+    ask();  // a small block did not fit: the chunk that the free memory allows
+  }
+  if (rc != CTC_OK) return rc;
   if ((rc = mol->ws_misc.ensure(tile_bytes(mol, (int)C, TP, Kcap), st)) != CTC_OK) return rc;
   TileBatch tb;
   tb.TP = TP;
