@@ -355,7 +355,7 @@ __global__ void atom_pair_nonzero_kernel(const double* __restrict__ D, int M, in
 // non-zero atom pair, and always for kb = 0 (the stage that initialises the
 // accumulators of a nu tile).  One block per tile; a 64-AO block with more
 // than kMaskAtoms distinct atoms is taken as non-zero.
-constexpr int kMaskAtoms = 16;
+constexpr int kMaskAtoms = 24;
 __global__ void __launch_bounds__(256)
     stage_mask_kernel(TileBatch tb, const int32_t* __restrict__ ao_atom, const uint8_t* __restrict__ nz,
                       int natom, uint32_t* __restrict__ mask, int mask_words) {
