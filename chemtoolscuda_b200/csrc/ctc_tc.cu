@@ -549,19 +549,21 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int nc = nt * kN + nrow0 + 8 * q;
-          nu[q] = nc < kt ? am[nc] : -1;
+          nu[q] = am[nc < kt ? nc : 0];
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) mu[q] = am[kb * kBK + k4 + q];
       };
+      // Padding (-1) reads D's first row or column: the A digits of padding
+      // columns and the scales of padding rows are zero.  (A condition on the
+      // load makes the compiler wait for each one before the next: contraction
+      // of the 530 000-point cube 74.8 ms with it, 67.7 ms without.)
       auto gather = [&](const int (&nu)[8], const int (&mu)[4], uint64_t (&w)[8][4]) {
 #pragma unroll
         for (int q = 0; q < 8; ++q)
 #pragma unroll
           for (int m = 0; m < 4; ++m)
-            w[q][m] = (nu[q] >= 0 && mu[m] >= 0)
-                          ? ldg_u64_hint(args.Dp + (int64_t)nu[q] * args.Mpad + mu[m], keep)
-                          : 0ull;
+            w[q][m] = ldg_u64_hint(args.Dp + (int64_t)max(nu[q], 0) * args.Mpad + max(mu[m], 0), keep);
       };
       int nu[8], mu[4];
       uint64_t w[8][4];
