@@ -131,9 +131,11 @@ struct TileBatch {
   int32_t* aomap = nullptr; // [C][Kcap] compact -> AO index, -1 for padding
   int32_t* order = nullptr; // [C] tiles, largest compact set first
   int32_t* counter = nullptr; // zero when the contraction starts
+  int32_t* parts = nullptr;   // work items per tile of the tensor-core contraction
   double* ao = nullptr;     // [C][nq][Kcap][TP] AO values and derivatives
 };
 constexpr int kKtAlign = 64;
+constexpr int kMaxParts = 8;
 
 }  // namespace ctc
 

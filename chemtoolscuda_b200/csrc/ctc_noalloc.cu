@@ -146,7 +146,8 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
     tb.k0 = tc.take<int32_t>((size_t)C * mol->nseg);
     tb.aomap = tc.take<int32_t>((size_t)C * tb.Kcap);
     tb.order = tc.take<int32_t>(C);
-    tb.counter = tc.take<int32_t>(1);
+    tb.counter = tc.take<int32_t>(2);
+    tb.parts = tb.counter + 1;
     tb.ao = tc.take<double>(ao_per_tile / sizeof(double) * (size_t)C);
     if (sort_end + tc.off > kNoAllocScratchBytes)
       return fail(CTC_ERR_INVALID, "ctc_eval_local_noalloc: internal scratch layout overflow");
@@ -166,7 +167,7 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
     screen_kernel<<<tb.C, kTileThreads, 0, st>>>(mol->d_segs, mol->nseg, tb, TP * plan.nqa, mol->d_stats,
                                                  mol->d_status);
     CTC_CUDA_TRY(cudaGetLastError());
-    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb);
+    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb, 148, 0.0);
     CTC_CUDA_TRY(cudaGetLastError());
     if ((rc = launch_ao_tiles(mol, tb, plan.deriv, st)) != CTC_OK) return rc;
     if ((rc = fp64_local_tiles(mol, plan, tb, prm, out, st)) != CTC_OK) return rc;

@@ -20,8 +20,9 @@
 //     the FP64 path).
 // The dropped products (i + j >= 5) are below 2^-40 of the row/column scale.
 //
-// Kernel roles (288 threads, one persistent CTA per SM taking the chunk's
-// tiles largest first from a launch-wide counter): warps 0-3 produce the
+// Kernel roles (288 threads, one persistent CTA per SM taking work items -- a
+// tile's nu slices dealt out to up to eight of them, tiles largest first -- from
+// a launch-wide counter): warps 0-3 produce the
 // operands of each K block (one thread issues the TMA loads of the five A
 // planes; all 128 threads gather the five D planes by compact index from the
 // packed copy of D and write them in the 64-byte-swizzled K-major layout),
@@ -303,14 +304,18 @@ __device__ __forceinline__ void contract_rows(const double* __restrict__ ao, int
   }
 }
 
+// adds the role's sums of one point to [sum][point] (stores the first slice's)
 template <int ROLE>
-__device__ __forceinline__ void store_role(double (*s_sums)[16], int lane, const double* acc) {
+__device__ __forceinline__ void add_role(double* ps, int lane, const double* acc, bool first) {
   constexpr int NS = role_nslot(ROLE);
   int i = 0;
 #pragma unroll
   for (int s = 0; s < NS; ++s)
 #pragma unroll
-    for (int rr = 0; rr < role_nrow(ROLE, s); ++rr, ++i) s_sums[lane][role_sum(ROLE, s, rr)] = acc[i];
+    for (int rr = 0; rr < role_nrow(ROLE, s); ++rr, ++i) {
+      double* d = ps + role_sum(ROLE, s, rr) * 32 + lane;
+      *d = first ? acc[i] : *d + acc[i];
+    }
 }
 
 // ------------------------------------------------------------------ preparation kernels
@@ -400,13 +405,19 @@ struct TcArgs {
   const int32_t* fexp;   // D row exponents
   const int32_t* eexp;   // A row exponents [C][128]
   int Mpad;
-  ctc_outputs out;
-  ctc_params prm;
   int32_t* status;
   // tile schedule: order[0..C) lists the chunk's tiles (largest compact K
   // first); tile_counter (zero at launch) hands them out to the CTAs
   const int32_t* order;
   int32_t* tile_counter;
+  // every tile's nu slices are dealt out to *parts work items (slice nt to item
+  // nt % parts, a divisor of kMaxParts); the sums of slice nt (512: 32 points x
+  // 16 or 128 points x 4) are added up at psum[(tile * slots + nt % kMaxParts) *
+  // 512], so the order of the additions does not depend on parts;
+  // tc_finish_kernel adds the slots
+  const int32_t* parts;
+  double* psum;
+  int slots;  // per tile: min(kMaxParts, slices of the widest tile)
   // limit of every pipeline wait, in SM cycles (kWaitCycles unless a caller
   // shortens it to exercise the timeout path)
   long long wait_cycles;
@@ -432,10 +443,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __shared__ __align__(8) uint64_t tile_full_bar[2], tile_empty_bar[2];
   __shared__ uint32_t tmem_base_sh;
   __shared__ int s_abort;
-  __shared__ int s_tile[2];
+  __shared__ int s_tile[2];  // work item: tile * parts + part
   __shared__ int s_epi_tile;
   __shared__ int s_epi_abort[2];
-  __shared__ double s_sums[32][16];
   __shared__ double s_cscale[2][kN];
 
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -470,6 +480,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_sh;
+  const int parts = *args.parts;
   const long long t_start = clock64();
   long long tr0 = 0, tr1 = 0, tr2 = 0;  // per-role trace counters
 
@@ -501,8 +512,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   };
   auto warp_abort = [&]() -> bool { return __any_sync(0xffffffffu, s_abort != 0); };
   // is stage j (= nu tile * nkb + K block) of tile t active?  (block-sparse D)
+  const bool sparse = args.stage_mask != nullptr;
   auto stage_on = [&](int t, int j) -> bool {
-    return !args.stage_mask ||
+    return !sparse ||
            ((__ldg(args.stage_mask + (int64_t)t * args.mask_words + (j >> 5)) >> (j & 31)) & 1u);
   };
 
@@ -531,21 +543,22 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
           s_abort = 1;
         } else {
           const int c = atomicAdd(args.tile_counter, 1);
-          next = c < tb.C ? args.order[c] : -1;
+          next = c < tb.C * parts ? args.order[c / parts] * parts + c % parts : -1;
         }
         s_tile[slot] = next;
         mbar_arrive(&tile_full_bar[slot]);
       }
-      const int t = read_tile_warp(i);
+      const int item = read_tile_warp(i);
       if (lane == 0) mbar_arrive(&tile_empty_bar[i & 1]);
-      if (t < 0 || warp_abort()) break;
+      if (item < 0 || warp_abort()) break;
+      const int t = item / parts, part = item % parts;
       const int kt = tb.kt[t];
       const int nkb = kt / kBK;
       const int nnt = (kt + kN - 1) / kN;
-      const int nst = nnt * nkb;
+      const int nst = nnt > part ? (nnt - part + parts - 1) / parts * nkb : 0;  // of this part
       const int32_t* am = tb.aomap + (int64_t)t * tb.Kcap;
       auto load_idx = [&](int j, int (&nu)[8], int (&mu)[4]) {
-        const int nt = j / nkb, kb = j - nt * nkb;
+        const int n = j / nkb, kb = j - n * nkb, nt = part + n * parts;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int nc = nt * kN + nrow0 + 8 * q;
@@ -569,7 +582,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       uint64_t w[8][4];
       // the tile's active stages in order (every stage unless D is block-sparse)
       auto next_on = [&](int j) -> int {
-        while (j < nst && !stage_on(t, j)) ++j;
+        if (!sparse) return j;
+        while (j < nst && !stage_on(t, (part + j / nkb * parts) * nkb + j % nkb)) ++j;
         return j;
       };
       int j = next_on(0);
@@ -649,14 +663,15 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
     const uint32_t idesc0 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRows >> 4) << 24);
     int it = 0, gnt = 0;  // stage and nu-tile counters across tiles
     for (int i = 0;; ++i) {
-      const int t = read_tile_warp(i);
+      const int item = read_tile_warp(i);
       if (lane == 0) mbar_arrive(&tile_empty_bar[i & 1]);
-      if (t < 0 || warp_abort()) break;
+      if (item < 0 || warp_abort()) break;
+      const int t = item / parts;
       const int kt = tb.kt[t];
       const int nkb = kt / kBK;
       const int nnt = (kt + kN - 1) / kN;
       bool failed = false;
-      for (int nt = 0; nt < nnt && !failed; ++nt, ++gnt) {
+      for (int nt = item % parts; nt < nnt && !failed; nt += parts, ++gnt) {
         const long long tw = clock64();
         if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar, (gnt & 1) ^ 1, args.wait_cycles))) {
           s_abort = 1;
@@ -742,8 +757,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
         mbar_arrive(&tile_empty_bar[i & 1]);
       }
       asm volatile("bar.sync 1, 128;\n" ::: "memory");
-      const int t = s_epi_tile;
-      if (t < 0) break;
+      const int item = s_epi_tile;
+      if (item < 0) break;
+      const int t = item / parts;
       const int kt = tb.kt[t];
       const int nnt = (kt + kN - 1) / kN;
       const int32_t* am = tb.aomap + (int64_t)t * tb.Kcap;
@@ -751,8 +767,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       // G = 2^(e_r + f_nu - 76) sum_L acc_L 2^(64 - 8 L); the drain below forms
       // sum_L acc_L 2^(32 - 8 L), so the row factor carries the remaining 2^-44
       const double rowscale = ldexp(1.0, args.eexp[(int64_t)t * kRows + r] - 44);
-      double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-      for (int nt = 0; nt < nnt; ++nt, ++gnt) {
+      for (int nt = item % parts; nt < nnt; nt += parts, ++gnt) {
         const int n0 = nt * kN;
         double* cs = s_cscale[gnt & 1];
         if (etid < kN) {
@@ -799,6 +814,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
         // (B) G of this nu tile complete in shared memory
         asm volatile("bar.sync 1, 128;\n" ::: "memory");
         const double* ao_nt = aop + (int64_t)n0 * PTS;
+        double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         if (NQA == 4) {
           switch (role) {
             case 0: contract_role<0, kEpiGroup>(ao_nt, ldq, sG, lane, nq_ao, stream, acc); break;
@@ -811,41 +827,20 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
           if (nq_ao == 1) contract_rows<1, 4>(ao_nt, ldq, sG, etid, stream, acc);
           else contract_rows<4, 2>(ao_nt, ldq, sG, etid, stream, acc);
         }
-        if (args.trace) {
-          // results of the contraction are complete when they are used
-          double chk = acc[0] + acc[1] + acc[2] + acc[3] + acc[4];
-          asm volatile("" : "+d"(chk));
-          tr2 += clock64() - tc0;
-        }
-      }
-      // (C) gather the per-point sums and finalise
-      asm volatile("bar.sync 1, 128;\n" ::: "memory");
-      const bool aborted = stop || s_abort != 0;
-      if (NQA == 4) {
-        switch (role) {
-          case 0: store_role<0>(s_sums, lane, acc); break;
-          case 1: store_role<1>(s_sums, lane, acc); break;
-          case 2: store_role<2>(s_sums, lane, acc); break;
-          default: store_role<3>(s_sums, lane, acc); break;
-        }
-        asm volatile("bar.sync 1, 128;\n" ::: "memory");
-        if (role == 0 && !aborted) {
-          const int64_t pi = (int64_t)t * tb.TP + lane;
-          const int64_t oidx = tb.out[pi];
-          if (oidx >= 0) {
-            if (finite_point(tb.xyz + 3 * pi)) finalize_point(s_sums[lane], 4, nq_ao, args.out, oidx, args.prm);
-            else nan_point(args.out, oidx);
+        double* ps = args.psum + ((int64_t)t * args.slots + nt % kMaxParts) * 512;
+        const bool first = nt < kMaxParts;
+        if (NQA == 4) {
+          switch (role) {
+            case 0: add_role<0>(ps, lane, acc, first); break;
+            case 1: add_role<1>(ps, lane, acc, first); break;
+            case 2: add_role<2>(ps, lane, acc, first); break;
+            default: add_role<3>(ps, lane, acc, first); break;
           }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) ps[q * kRows + etid] = first ? acc[q] : ps[q * kRows + etid] + acc[q];
         }
-      } else if (!aborted) {
-        const int64_t pi = (int64_t)t * tb.TP + etid;
-        const int64_t oidx = tb.out[pi];
-        double s16[16];
-        for (int q = 0; q < 16; ++q) s16[q] = q < 4 ? acc[q] : 0.0;
-        if (oidx >= 0) {
-          if (finite_point(tb.xyz + 3 * pi)) finalize_point(s16, 1, nq_ao, args.out, oidx, args.prm);
-          else nan_point(args.out, oidx);
-        }
+        if (args.trace) tr2 += clock64() - tc0;
       }
     }
     if (args.trace && etid == 0) {
@@ -866,6 +861,30 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem));
   }
+}
+
+// Adds the slots of every tile's sums in order and finishes its points.
+template <int NQA>
+__global__ void __launch_bounds__(128)
+    tc_finish_kernel(TileBatch tb, const double* __restrict__ psum, int slots, ctc_outputs out, ctc_params prm) {
+  constexpr int PTS = kRows / NQA, NS = NQA == 4 ? 16 : 4;
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = gid / PTS;
+  if (t >= tb.C) return;
+  const int p = (int)(gid % PTS);
+  const int64_t oidx = tb.out[gid];
+  if (oidx < 0) return;
+  const int used = min(kMaxParts, (tb.kt[t] + kN - 1) / kN);
+  double s[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) s[q] = 0.0;
+  for (int k = 0; k < used; ++k) {
+    const double* ps = psum + (t * slots + k) * 512 + p;
+#pragma unroll
+    for (int q = 0; q < NS; ++q) s[q] += ps[q * PTS];
+  }
+  if (finite_point(tb.xyz + 3 * gid)) finalize_point(s, NQA, tb.nq, out, oidx, prm);
+  else nan_point(out, oidx);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
@@ -930,6 +949,8 @@ struct TcWorkspace {
   int32_t* eexp;
   uint32_t* mask;  // active K stages per tile (mask_words each), block-sparse D only
   int mask_words;
+  double* psum;    // partial sums, slots x 512 per tile
+  int slots;
 };
 
 int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t st, TcWorkspace* w) {
@@ -944,6 +965,7 @@ int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t 
   const int nbmax = tb.Kcap / kBK;
   const int mask_words = mol->d_nzpair ? (nbmax * nbmax + 31) / 32 : 0;
   const size_t o_mask = take(sizeof(uint32_t) * (size_t)tb.C * mask_words);
+  const size_t o_psum = take(sizeof(double) * 512 * (size_t)tb.C * std::min(kMaxParts, tb.Kcap / kN));
   int rc = mol->ws_sl.ensure(off, st);
   if (rc != CTC_OK) return rc;
   char* base = (char*)mol->ws_sl.p;
@@ -951,6 +973,8 @@ int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t 
   w->eexp = (int32_t*)(base + o_eexp);
   w->mask = mask_words ? (uint32_t*)(base + o_mask) : nullptr;
   w->mask_words = mask_words;
+  w->psum = (double*)(base + o_psum);
+  w->slots = std::min(kMaxParts, tb.Kcap / kN);
   return CTC_OK;
 }
 
@@ -993,7 +1017,7 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   if (cr != CUDA_SUCCESS) return fail(CTC_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)cr));
   int num_sms = 0;
   if ((rc = device_sm_count(&num_sms)) != CTC_OK) return rc;
-  const int grid = std::min(tb.C, num_sms);
+  const int grid = (int)std::min<int64_t>((int64_t)tb.C * kMaxParts, num_sms);
   TcArgs a;
   a.tb = tb;
   a.nqa = plan.nqa;
@@ -1001,10 +1025,11 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   a.fexp = (const int32_t*)mol->d_Dscale;
   a.eexp = w.eexp;
   a.Mpad = mol->Mpad;
-  a.out = *out;
-  a.prm = *prm;
   a.status = mol->d_status;
   a.order = tb.order;
+  a.parts = tb.parts;
+  a.psum = w.psum;
+  a.slots = w.slots;
   a.tile_counter = tb.counter;
   a.trace = nullptr;
   a.wait_cycles = mol->wait_cycles > 0 ? (long long)mol->wait_cycles : kWaitCycles;
@@ -1027,6 +1052,13 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   if (plan.nqa == 4) tc_tile_kernel<4><<<grid, kThreadsTc, kSmemTc, st>>>(amap, a);
   else tc_tile_kernel<1><<<grid, kThreadsTc, kSmemTc, st>>>(amap, a);
   CTC_CUDA_TRY(cudaGetLastError());
+  {
+    const unsigned g = (unsigned)(((int64_t)tb.C * tb.TP + 127) / 128);
+    if (plan.nqa == 4) tc_finish_kernel<4><<<g, 128, 0, st>>>(tb, w.psum, a.slots, *out, *prm);
+    else tc_finish_kernel<1><<<g, 128, 0, st>>>(tb, w.psum, a.slots, *out, *prm);
+    CTC_CUDA_TRY(cudaGetLastError());
+    mol->host_launches += 1;
+  }
   if (trace_on) {
     std::vector<long long> tr((size_t)8 * grid);
     std::vector<int32_t> kt(tb.C);

@@ -416,21 +416,50 @@ __global__ void __launch_bounds__(kTileThreads)
 }
 
 // The chunk's tiles, largest compact set first (counting sort by kt / 64; the
-// order within a bin is free), and the chunk's tile counter set to zero.  Both
-// contractions and the tensor-core path's AO kernel take the tiles in this
-// order, so the last tiles of a launch are the cheapest.  One block: ~4 us at
-// 2 000 tiles, where a radix sort of the counts took ~8 us and two launches.
+// order within a bin is free), the chunk's tile counter set to zero, and the
+// work items per tile of the tensor-core contraction.  The FP64 contraction and
+// the tensor-core path's AO kernel take the tiles in this order, so the last
+// tiles of a launch are the cheapest.  One block: ~4 us at 2 000 tiles, where a
+// radix sort of the counts took ~8 us and two launches.
+//
+// A tile's digit planes (640 bytes per function) are read once for every 64
+// functions and D by every tile, so the contraction wants the planes of the
+// tiles in flight and D in L2: with `parts` items per tile the SMs work on 1 /
+// parts as many tiles.  parts is the smallest power of two for which the planes
+// and D (8 M^2 bytes, or what the tiles use of it) stay below kL2Bytes, and at
+// least what gives every SM four items.  (One item per tile: contraction of the
+// 530 000-point cube of 200 atoms 67.7 ms, with parts 56.6; 640-atom sparse cube
+// 153 and 136; 300 000 host points 16.2 and 14.5.)
 constexpr int kOrderThreads = 1024;
-__global__ void __launch_bounds__(kOrderThreads) tile_order_kernel(TileBatch tb) {
+constexpr double kL2Bytes = 96e6;
+__global__ void __launch_bounds__(kOrderThreads) tile_order_kernel(TileBatch tb, int sms, double d_bytes) {
   using Scan = cub::BlockScan<int, kOrderThreads>;
   __shared__ typename Scan::TempStorage tmp;
   __shared__ int s_bin[kOrderThreads];
+  __shared__ unsigned long long s_kt;
   s_bin[threadIdx.x] = 0;
-  if (threadIdx.x == 0) *tb.counter = 0;
+  if (threadIdx.x == 0) {
+    *tb.counter = 0;
+    s_kt = 0;
+  }
   __syncthreads();
   auto bin = [&](int t) { return kOrderThreads - 1 - min(tb.kt[t] / kKtAlign, kOrderThreads - 1); };
-  for (int t = threadIdx.x; t < tb.C; t += kOrderThreads) atomicAdd(&s_bin[bin(t)], 1);
+  unsigned long long kt = 0;
+  for (int t = threadIdx.x; t < tb.C; t += kOrderThreads) {
+    atomicAdd(&s_bin[bin(t)], 1);
+    kt += tb.kt[t];
+  }
+  for (int o = 16; o > 0; o >>= 1) kt += __shfl_xor_sync(0xffffffffu, kt, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&s_kt, kt);
   __syncthreads();
+  if (threadIdx.x == 0) {
+    const double mean = (double)s_kt / tb.C, d = fmin(d_bytes, 0.6 * kL2Bytes);
+    int parts = 1;
+    while (parts < kMaxParts && ((double)min(sms, tb.C * parts) / parts * 640.0 * mean + d > kL2Bytes ||
+                                 (int64_t)tb.C * parts < 4 * sms))
+      parts *= 2;
+    *tb.parts = parts;
+  }
   int first;
   Scan(tmp).ExclusiveSum(s_bin[threadIdx.x], first);
   __syncthreads();
@@ -466,7 +495,7 @@ size_t tile_bytes(const ctc_molecule* mol, int C, int TP, int Kcap_) {
   add(sizeof(int32_t) * (size_t)C * mol->nseg);
   add(sizeof(int32_t) * (size_t)C * Kcap);
   add(sizeof(int32_t) * C);
-  add(sizeof(int32_t));
+  add(2 * sizeof(int32_t));
   return b + 256;
 }
 
@@ -623,6 +652,8 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   }
   if (rc != CTC_OK) return rc;
   if ((rc = mol->ws_misc.ensure(tile_bytes(mol, (int)C, TP, Kcap), st)) != CTC_OK) return rc;
+  int nsm = 148;
+  if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   TileBatch tb;
   tb.TP = TP;
   tb.Kcap = Kcap;
@@ -639,7 +670,8 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     tb.k0 = cv.take<int32_t>((size_t)C * mol->nseg);
     tb.aomap = cv.take<int32_t>((size_t)C * tb.Kcap);
     tb.order = cv.take<int32_t>(C);
-    tb.counter = cv.take<int32_t>(1);
+    tb.counter = cv.take<int32_t>(2);
+    tb.parts = tb.counter + 1;
   }
   for (int64_t t0 = 0; t0 < ntiles; t0 += C) {
     tb.C = (int)std::min<int64_t>(C, ntiles - t0);
@@ -647,7 +679,7 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     screen_kernel<<<tb.C, kTileThreads, 0, st>>>(mol->d_segs, mol->nseg, tb, rows, mol->d_stats,
                                                  mol->d_status);
     CTC_CUDA_TRY(cudaGetLastError());
-    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb);
+    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb, nsm, 8.0 * mol->M * mol->M);
     CTC_CUDA_TRY(cudaGetLastError());
     {
       ProfScope ps(mol, 1, st);
