@@ -20,7 +20,7 @@
 // 2. Rate.  One persistent CTA per SM with separate warps for the loads, the
 //    matrix instructions and the epilogue, so that index loads, gathers of D
 //    and the epilogue's AO reads run beside the matrix pipe: 4 producer warps
-//    (cp.async; A rows and D gathered by compact index, 3 stages of 32 mu),
+//    (A rows by bulk copies, D gathered by compact index; 3 stages of 32 mu),
 //    8 matrix warps, 4 epilogue warps working on the previous slice.
 //
 // Measured (one B200, device time of the kernel; before: one CTA per tile whose
@@ -54,7 +54,7 @@ constexpr int kFAStage = kFK * kFALd, kFBStage = kFK * kFBLd;
 constexpr int kFThreads = 512;     // warps 0-3 producers, 4-7 epilogue, 8-15 matrix
 constexpr size_t kFSmem = sizeof(double) * (kFStages * (kFAStage + kFBStage) + kFN * kFGLd);
 constexpr int kFSums = 19;         // per-point sums of the widest epilogue
-constexpr int kFProducerRegs = 56, kFEpilogueRegs = 152, kFMatrixRegs = 152;
+constexpr int kFProducerRegs = 112, kFEpilogueRegs = 128, kFMatrixRegs = 136;
 static_assert(128 * kFProducerRegs + 128 * kFEpilogueRegs + 256 * kFMatrixRegs <= kFThreads * 128,
               "register split above the launch's total");
 static_assert(kKtAlign % kFN == 0 && kFN % kFK == 0, "tile K alignment");
@@ -91,16 +91,13 @@ struct Fp64Args {
   int natom;
 };
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem)), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
-  const int sz = valid ? 8 : 0;  // 0: the destination is zero-filled
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(sz));
-}
-// the barrier receives this thread's arrival once its earlier cp.async have landed
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+// bytes (a multiple of 16; both addresses 16-byte aligned) global -> shared,
+// counted on bar
+__device__ __forceinline__ void bulk_copy(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   smem_u32(smem)),
+               "l"(gmem), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
@@ -234,7 +231,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
   double* sA = fsmem;
   double* sB = fsmem + kFStages * kFAStage;
   double* sG = fsmem + kFStages * (kFAStage + kFBStage);
-  __shared__ __align__(8) uint64_t full_bar[kFStages], empty_bar[kFStages], gfull_bar, gempty_bar, gwide_bar;
+  __shared__ __align__(8) uint64_t full_bar[kFStages], tma_bar[kFStages], empty_bar[kFStages], gfull_bar, gempty_bar, gwide_bar;
   __shared__ double s_sums[32][kFSums + 1];
   __shared__ int s_abort, s_epi_abort;
 
@@ -242,7 +239,8 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kFStages; ++s) {
-      mbar_init(&full_bar[s], 128);
+      mbar_init(&full_bar[s], 64);
+      mbar_init(&tma_bar[s], 2);
       mbar_init(&empty_bar[s], 8);
     }
     mbar_init(&gfull_bar, 8);
@@ -259,66 +257,116 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
   if (warp < 4) {
     // ---------------- producers
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kFProducerRegs));
-    const int tid = threadIdx.x;
-    const int arow = (tid & 63) * 2, ak = tid >> 6;  // A: row pair, mu = ak + 2 i
-    const int bcol = tid & 63, bk = tid >> 6;        // B: nu column, mu = bk + 2 i
-    // the row pair's quantity (kFForce2: the second row block is quantity 10)
-    const int aq = MODE == kFForce2 ? (arow / PTS ? 10 : 0) : (MODE == kFLocal4 ? arow / PTS : 0);
-    const int nrow = (tid & 15) * 2, nk0 = tid >> 4;  // narrow A stage: row pair, mu = nk0 + 8 i
-    int it = 0;
-    bool stop = false;
-    for (int i = 0; !stop; ++i) {
-      const int t = fturn(tb, i);
-      if (t < 0) break;
-      const int nk = (tb.ktrue[t] + kFK - 1) / kFK;  // columns beyond ktrue are zero
-      const int nn = (nk * kFK + kFN - 1) / kFN;
-      const int32_t* am = tb.aomap + (int64_t)t * tb.Kcap;
-      const double* A = tb.ao + (int64_t)t * nq_ao * ldq;
-      const double* Aw = A + aq * ldq + arow % PTS;
-      int idx = nk > 0 ? am[lane] : -1;  // this stage's 32 mu, one per lane
-      for (int nt = 0; nt < nn && !stop; ++nt) {
-        const FSlice fs = fslice<MODE>(nt, nk, tri, nq_ao);
-        const int nu = am[nt * kFN + bcol];  // -1 beyond ktrue (padded to 64)
-        for (int kb = 0; kb < fs.total; ++kb, ++it) {
-          const int s = it % kFStages;
-          // next stage's indices (the next slice starts again at mu 0)
-          const int nxt = am[(kb + 1 < fs.total ? kb + 1 : 0) * kFK + lane];
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / kFStages) & 1) ^ 1, args.wait_cycles))) {
-            s_abort = 1;
-            stop = true;
-            break;
-          }
-          double* a = sA + s * kFAStage;
-          double* b = sB + s * kFBStage;
-          const int k0 = kb * kFK;
-          if (!NARROW_ONLY && kb < fs.wide) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int kk = ak + 2 * j;
-              cp_async16(a + kk * kFALd + arow, Aw + (int64_t)(k0 + kk) * PTS);
-            }
-          } else if (HAS_NARROW) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int kk = nk0 + 8 * j;
-              cp_async16(a + kk * kFALd + nrow, A + (int64_t)(k0 + kk) * PTS + nrow);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int kk = bk + 2 * j;
-            const int mu = __shfl_sync(0xffffffffu, idx, kk);
-            const bool v = mu >= 0 && nu >= 0;
-            cp_async8(b + kk * kFBLd + bcol, args.D + (v ? (int64_t)mu * args.Mpad + nu : 0), v);
-          }
-          cp_async_arrive(&full_bar[s]);
-          idx = nxt;
-        }
+    // Warps 0-1 take the even stages of the CTA's sequence, warps 2-3 the odd
+    // ones.  A thread gathers one nu column of D for 16 + 16 mu into registers,
+    // the loads of its next stage in flight while this one waits for its slot;
+    // the A rows are bulk copies of one (mu, quantity) run of points each.
+    // (cp.async for both takes the L1 a cycle per lane: ~1.7 K for the D block
+    // and ~2 K for the A rows of a stage whose matrix instructions take 4.1 K
+    // with all rows and 1 K with the phi rows.)
+    const int pair = warp >> 1, ptid = threadIdx.x & 63;
+    const int khalf = warp & 1;  // bulk copies: mu 16 khalf .. + 15 by this warp
+    struct Cur {
+      int i, t, nk, nn, nt, kb, total, wide;
+    };
+    auto open_tile = [&](Cur& c) {  // first stage of the next tile that has any
+      for (;; ++c.i) {
+        c.t = fturn(tb, c.i);
+        if (c.t < 0) return;
+        c.nk = (tb.ktrue[c.t] + kFK - 1) / kFK;  // columns beyond ktrue are zero
+        c.nn = (c.nk * kFK + kFN - 1) / kFN;
+        if (c.nn > 0) break;
       }
-      if (__any_sync(0xffffffffu, s_abort != 0)) break;
+      const FSlice fs = fslice<MODE>(0, c.nk, tri, nq_ao);
+      c.nt = c.kb = 0;
+      c.total = fs.total;
+      c.wide = fs.wide;
+    };
+    auto advance = [&](Cur& c) {
+      if (c.t < 0 || ++c.kb < c.total) return;
+      c.kb = 0;
+      if (++c.nt < c.nn) {
+        const FSlice fs = fslice<MODE>(c.nt, c.nk, tri, nq_ao);
+        c.total = fs.total;
+        c.wide = fs.wide;
+        return;
+      }
+      ++c.i;
+      open_tile(c);
+    };
+    double v[kFK];
+    unsigned ok = 0;  // mu of the stage that are not padding
+    bool nu_ok = false;
+    auto load_idx = [&](const Cur& c, int& mu, int& nu) {
+      const int32_t* am = tb.aomap + (int64_t)c.t * tb.Kcap;
+      mu = am[c.kb * kFK + lane];
+      nu = am[c.nt * kFN + ptid];  // -1 beyond ktrue (padded to 64)
+    };
+    // loads without a condition (clamped index; the value is dropped later): a
+    // condition on each makes the compiler wait for one before the next
+    auto gather = [&](int mu, int nu) {
+      ok = __ballot_sync(0xffffffffu, mu >= 0);
+      nu_ok = nu >= 0;
+      const int m = max(mu, 0);
+      const double* d = args.D + max(nu, 0);
+#pragma unroll
+      for (int k = 0; k < kFK; ++k) v[k] = __ldg(d + (int64_t)__shfl_sync(0xffffffffu, m, k) * args.Mpad);
+    };
+    int last_issue[kFStages];
+#pragma unroll
+    for (int s = 0; s < kFStages; ++s) last_issue[s] = -1;
+    Cur cur{};
+    open_tile(cur);
+    if (pair) advance(cur);
+    if (cur.t >= 0) {
+      int mu, nu;
+      load_idx(cur, mu, nu);
+      gather(mu, nu);
     }
-    // no copy may land after the CTA has left
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    for (int it = pair; cur.t >= 0; it += 2) {
+      Cur nxt = cur;
+      advance(nxt);
+      advance(nxt);
+      int mu = -1, nu = -1;
+      if (nxt.t >= 0) load_idx(nxt, mu, nu);
+      const int s = it % kFStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / kFStages) & 1) ^ 1, args.wait_cycles))) {
+        s_abort = 1;
+        break;
+      }
+      double* a = sA + s * kFAStage;
+      double* b = sB + s * kFBStage;
+      {
+        const double* A = tb.ao + (int64_t)cur.t * nq_ao * ldq + (int64_t)cur.kb * kFK * PTS;
+        const bool wide = !NARROW_ONLY && cur.kb < cur.wide;
+        constexpr int NRUN = MODE == kFLocal4 ? 4 : (MODE == kFForce2 ? 2 : 1);  // quantities of a wide stage
+        const int runs = wide ? NRUN : 1;
+        if (lane == 0) mbar_arrive_expect_tx(&tma_bar[s], 16 * runs * PTS * 8);
+        __syncwarp();
+        for (int x = lane; x < 16 * runs; x += 32) {
+          const int kk = 16 * khalf + x / runs, r = x % runs;
+          const int q = MODE == kFForce2 ? 10 * r : r;
+          bulk_copy(a + kk * kFALd + r * PTS, A + q * ldq + (int64_t)kk * PTS, PTS * 8, &tma_bar[s]);
+        }
+#pragma unroll
+        for (int z = 0; z < kFStages; ++z)
+          if (z == s) last_issue[z] = it;
+      }
+#pragma unroll
+      for (int k = 0; k < kFK; ++k) b[k * kFBLd + ptid] = (nu_ok && ((ok >> k) & 1u)) ? v[k] : 0.0;
+      mbar_arrive(&full_bar[s]);
+      if (nxt.t >= 0) gather(mu, nu);
+      cur = nxt;
+    }
+    // No copy may land after the CTA has left.  After a normal end the matrix
+    // warps wait for every one; after a timeout some may be on their way, and
+    // each slot's last copies are waited for with the full limit (a slot that the
+    // other pair has used since is past that phase: its wait runs out).
+    if (s_abort) {
+#pragma unroll
+      for (int s = 0; s < kFStages; ++s)
+        if (last_issue[s] >= 0) mbar_wait(&tma_bar[s], (last_issue[s] / kFStages) & 1);
+    }
   } else if (warp >= 8) {
     // ---------------- matrix warps
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kFMatrixRegs));
@@ -345,7 +393,9 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
         }
         for (int kb = 0; kb < fs.total; ++kb, ++it) {
           const int s = it % kFStages;
-          if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], (it / kFStages) & 1, args.wait_cycles))) {
+          const uint32_t ph = (it / kFStages) & 1;
+          const bool ready = mbar_wait(&full_bar[s], ph, args.wait_cycles) && mbar_wait(&tma_bar[s], ph, args.wait_cycles);
+          if (!__all_sync(0xffffffffu, ready)) {
             s_abort = 1;
             stop = true;
             break;
@@ -441,7 +491,6 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
     }
   } else {
     // ---------------- epilogue warps
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kFEpilogueRegs));
     const int role = warp - 4;
     const int etid = role * 32 + lane;
     int gs = 0;
