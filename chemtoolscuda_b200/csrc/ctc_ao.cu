@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(kAoThreads, 3)
 }
 
 // Digit planes of the tile rows (ctc_split.cuh) with the exponents found by
-// ao_tile_kernel.  One block per tile, the tiles taken in the chunk's order
+// ao_tile_kernel, columns in the order of the tile's quads of AOs (TileBatch::ksrc;
+// places without a compact AO get zeros).  One block per tile, the tiles taken in the chunk's order
 // (largest compact K first) when one is given.  Work items are (32-row
 // group, 32-column chunk); the block's warps take them in turn: a warp reads
 // one 256-byte line per column (32 consecutive rows = points of one
@@ -240,14 +241,15 @@ __global__ void __launch_bounds__(kSliceThreads, 2)
     slice_rows_kernel(TileBatch tb, int nqa, const int32_t* __restrict__ eexp,
                       int8_t* __restrict__ planes, const int32_t* __restrict__ order) {
   const int t = order ? order[blockIdx.x] : blockIdx.x;
-  const int kt = tb.kt[t];
+  const int kp = tb.kp[t];
   const int TP = tb.TP;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ld_q = (int64_t)TP * tb.Kcap;
   const double* A = tb.ao + (int64_t)t * tb.nq * ld_q;
+  const int32_t* ksrc = tb.ksrc + (int64_t)t * tb.Kpcap;
   const int rows = split_tile_rows(TP, nqa);
-  int8_t* P = planes + (int64_t)t * kSplitPlanesA * rows * tb.Kcap;
-  const int nitem = (rows / 32) * (kt / 32);  // warp-sized items
+  int8_t* P = planes + (int64_t)t * kSplitPlanesA * rows * tb.Kpcap;
+  const int nitem = (rows / 32) * (kp / 32);  // warp-sized items
   for (int it = warp; it < nitem; it += kSliceThreads / 32) {
     const int rg = it % (rows / 32), c = it / (rows / 32);
     const int r = rg * 32 + lane;             // tile row
@@ -255,13 +257,15 @@ __global__ void __launch_bounds__(kSliceThreads, 2)
     const int q = nqa == 4 ? rg % 4 : 0;      // quantity
     const int p = nqa == 4 ? blk * 32 + lane : r;  // point
     const double f = split_row_factor(eexp[(int64_t)t * rows + r], kFixedBitsA);
-    const double* col = A + q * ld_q + p + (int64_t)(c * 32) * TP;
+    const double* col = A + q * ld_q + p;
+    const int src = ksrc[c * 32 + lane];
+    const unsigned used = __ballot_sync(0xffffffffu, src >= 0);
     double v[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __ldg(col + (int64_t)i * TP);
-    write_row_digits32([&](int i) { return v[i]; }, f,
-                       P + (int64_t)blk * kSplitPlanesA * kSplitRows * tb.Kcap, r % kSplitRows,
-                       tb.Kcap, c * 32);
+    for (int i = 0; i < 32; ++i) v[i] = __ldg(col + (int64_t)max(__shfl_sync(0xffffffffu, src, i), 0) * TP);
+    write_row_digits32([&](int i) { return (used >> i) & 1u ? v[i] : 0.0; }, f,
+                       P + (int64_t)blk * kSplitPlanesA * kSplitRows * tb.Kpcap, r % kSplitRows,
+                       tb.Kpcap, c * 32);
   }
 }
 

@@ -129,6 +129,12 @@ struct TileBatch {
   int32_t* segs = nullptr;  // [C][nseg] significant segment ids
   int32_t* k0 = nullptr;    // [C][nseg] compact offset of each significant segment
   int32_t* aomap = nullptr; // [C][Kcap] compact -> AO index, -1 for padding
+  // K side of the tensor-core contraction: the quads of four consecutive AOs
+  // (ao / 4) that hold a compact AO, ascending, padded to 64 AOs
+  int Kpcap = 0;            // capacity in AOs (0: not formed)
+  int32_t* kp = nullptr;    // [C] AOs of the tile's quads, padded to 64
+  int32_t* kq = nullptr;    // [C][Kpcap / 4] quad indices
+  int32_t* ksrc = nullptr;  // [C][Kpcap] compact index of each place, -1: zero column
   int32_t* order = nullptr; // [C] tiles, largest compact set first
   int32_t* counter = nullptr; // zero when the contraction starts
   int32_t* parts = nullptr;   // work items per tile of the tensor-core contraction
@@ -162,7 +168,8 @@ struct ctc_molecule {
   int32_t* d_ao_atom = nullptr;
   double* d_D = nullptr;                     // Mpad x Mpad, zero padded
   int32_t* d_sym = nullptr;                  // 1: D is symmetric (set_symmetry_flag)
-  // split-precision copy of D (4 int8 byte planes, row scales)
+  // split-precision copy of D: per row and quad of four columns the plane words
+  // of digits 0-3 (16 bytes), then those of digit 4 (4 bytes); row scales
   int8_t* d_Dsl = nullptr;
   double* d_Dscale = nullptr;
   bool dsl_valid = false;
@@ -204,7 +211,7 @@ int launch_ao_tiles_weighted(const ctc_molecule* mol, const TileBatch& tb, const
                              const double* v_grad, cudaStream_t st);
 // The plain form, and in the same kernel the int8 digit planes of the tile rows
 // (nqa = 4: 32 points x {phi, d phi}; nqa = 1: 128 points x phi) with one
-// exponent per row, for the tensor-core split path: planes [C][5][128][Kcap],
+// exponent per row, for the tensor-core split path: planes [C][5][128][Kpcap],
 // eexp [C][128].
 // order (optional) lists the tiles in the order the CTAs take them.
 int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int deriv, int nqa,

@@ -97,7 +97,7 @@ int eval_local(ctc_molecule* mol, const PointSrc& src, int64_t n, int precision,
         mol->host_launches += 1;
         return r;
       },
-      precision == CTC_PREC_TC_SPLIT ? &sliced_ao : nullptr, rows);
+      precision == CTC_PREC_TC_SPLIT ? &sliced_ao : nullptr, rows, precision == CTC_PREC_TC_SPLIT);
   if (rc != CTC_OK) return rc;
   // kernels report failures (bounded-wait timeouts of the tensor-core
   // kernels, a tile beyond the workspace capacity) through the status word:

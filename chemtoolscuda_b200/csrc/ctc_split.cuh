@@ -29,7 +29,7 @@ constexpr int kSplitRows = 128;   // rows of one block of a tile operand (MMA M)
 
 // A tile of TP points with nqa row quantities (nqa = 4: phi and grad phi;
 // nqa = 1: phi) has nqa * TP operand rows, stored in blocks of 128 rows:
-// digit planes [tile][block][5][128][Kcap], row exponents [tile][rows].
+// digit planes [tile][block][5][128][Kpcap], row exponents [tile][rows].
 // With nqa = 4 point p's quantity q is row (p / 32) * 128 + q * 32 + p % 32,
 // so every block holds 32 points x 4 quantities; with nqa = 1 row = point.
 __host__ __device__ constexpr int split_tile_rows(int TP, int nqa) { return TP * nqa; }
@@ -98,13 +98,13 @@ __device__ __forceinline__ void transpose_bytes4x4(uint32_t a, uint32_t b, uint3
 }
 
 // Writes 32 consecutive K entries of one tile row into the five A planes
-// [plane][row][Kcap] (32 bytes per plane): x(i) returns the row's value at
+// [plane][row][ld] (32 bytes per plane): x(i) returns the row's value at
 // K index k0 + i, f = split_row_factor(e, kFixedBitsA) of the row.  The four
 // most significant digits go through pack_digits, the fifth is the balanced
 // low byte.
 template <class F>
 __device__ __forceinline__ void write_row_digits32(F x, double f, int8_t* __restrict__ P, int row,
-                                                   int64_t Kcap, int k0) {
+                                                   int64_t ld, int k0) {
   uint32_t pw[kSplitPlanesA][8];
 #pragma unroll
   for (int g = 0; g < 8; ++g) {
@@ -124,7 +124,7 @@ __device__ __forceinline__ void write_row_digits32(F x, double f, int8_t* __rest
   }
 #pragma unroll
   for (int p = 0; p < kSplitPlanesA; ++p) {
-    uint4* dst = reinterpret_cast<uint4*>(P + ((int64_t)p * kSplitRows + row) * Kcap + k0);
+    uint4* dst = reinterpret_cast<uint4*>(P + ((int64_t)p * kSplitRows + row) * ld + k0);
     dst[0] = make_uint4(pw[p][0], pw[p][1], pw[p][2], pw[p][3]);
     dst[1] = make_uint4(pw[p][4], pw[p][5], pw[p][6], pw[p][7]);
   }

@@ -114,9 +114,16 @@ __device__ __forceinline__ void tma_load_2d_hint(void* dst, const CUtensorMap* m
       : "memory");
 }
 
-__device__ __forceinline__ uint64_t ldg_u64_hint(const uint64_t* p, uint64_t policy) {
-  uint64_t v;
-  asm("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;\n" : "=l"(v) : "l"(p), "l"(policy));
+__device__ __forceinline__ uint4 ldg_u128_hint(const uint4* p, uint64_t policy) {
+  uint4 v;
+  asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;\n"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p), "l"(policy));
+  return v;
+}
+__device__ __forceinline__ uint32_t ldg_u32_hint(const uint32_t* p, uint64_t policy) {
+  uint32_t v;
+  asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;\n" : "=r"(v) : "l"(p), "l"(policy));
   return v;
 }
 
@@ -319,10 +326,11 @@ __device__ __forceinline__ void add_role(double* ps, int lane, const double* acc
 }
 
 // ------------------------------------------------------------------ preparation kernels
-// D (Mpad x Mpad, symmetric) -> one 64-bit word of five digits per element
-// (pack_digits5), exponent per row.
-__global__ void slice_d_kernel(const double* __restrict__ D, int Mpad, uint64_t* __restrict__ Dp,
-                               int32_t* __restrict__ fexp) {
+// D (Mpad x Mpad, symmetric) -> per row and quad of four columns the plane words
+// of its digits (words: digits 0-3, each word the four columns' bytes; low: digit
+// 4), exponent per row.
+__global__ void slice_d_kernel(const double* __restrict__ D, int Mpad, uint4* __restrict__ words,
+                               uint32_t* __restrict__ low, int32_t* __restrict__ fexp) {
   const int row = blockIdx.x;
   const double* d = D + (int64_t)row * Mpad;
   double m = 0.0;
@@ -340,8 +348,17 @@ __global__ void slice_d_kernel(const double* __restrict__ D, int Mpad, uint64_t*
   const int e = scale_exponent(red[0]);
   if (threadIdx.x == 0) fexp[row] = e;
   const double f = split_row_factor(e, kFixedBitsD);
-  for (int k = threadIdx.x; k < Mpad; k += blockDim.x)
-    Dp[(int64_t)row * Mpad + k] = pack_digits5(rint_i64(d[k] * f));
+  for (int q = threadIdx.x; q < Mpad / 4; q += blockDim.x) {
+    uint64_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = pack_digits5(rint_i64(d[4 * q + i] * f));
+    uint32_t pl[4];
+    transpose_bytes4x4((uint32_t)w[0], (uint32_t)w[1], (uint32_t)w[2], (uint32_t)w[3], pl);
+    const int64_t o = (int64_t)row * (Mpad / 4) + q;
+    words[o] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+    low[o] = (uint32_t)(w[0] >> 32) | (uint32_t)(w[1] >> 32) << 8 | (uint32_t)(w[2] >> 32) << 16 |
+             (uint32_t)(w[3] >> 32) << 24;
+  }
 }
 
 // Atom pairs with a non-zero element of D: nz[a * natom + b] = 1 for every
@@ -355,44 +372,50 @@ __global__ void atom_pair_nonzero_kernel(const double* __restrict__ D, int M, in
   if (D[(int64_t)i * Mpad + j] != 0.0) nz[(int64_t)ao_atom[i] * natom + ao_atom[j]] = 1;
 }
 
-// Active K stages of each tile: bit nt * nb + kb of tile t's mask is set when
-// the D block of nu block nt and mu block kb (64 compact AOs each) has a
+// Active K stages of each tile: bit nt * nbk + kb of tile t's mask is set when
+// the D block of nu block nt (64 compact AOs) and mu block kb (16 quads) has a
 // non-zero atom pair, and always for kb = 0 (the stage that initialises the
 // accumulators of a nu tile).  One block per tile; a 64-AO block with more
 // than kMaskAtoms distinct atoms is taken as non-zero.
-constexpr int kMaskAtoms = 24;
+constexpr int kMaskAtoms = 22;
+constexpr int kMaskBlocks = 256;  // per side; later blocks are taken as non-zero
 __global__ void __launch_bounds__(256)
     stage_mask_kernel(TileBatch tb, const int32_t* __restrict__ ao_atom, const uint8_t* __restrict__ nz,
                       int natom, uint32_t* __restrict__ mask, int mask_words) {
-  __shared__ int s_at[256][kMaskAtoms + 1];  // per 64-AO block: count, then atoms
+  __shared__ int s_at[2][kMaskBlocks][kMaskAtoms + 1];  // per 64-AO block of either side: count, then atoms
   const int t = blockIdx.x;
-  const int nb = tb.kt[t] / 64;
+  const int nb = tb.kt[t] / 64, nbk = tb.kp[t] / 64;
   const int32_t* am = tb.aomap + (int64_t)t * tb.Kcap;
+  const int32_t* ks = tb.ksrc + (int64_t)t * tb.Kpcap;
   uint32_t* mk = mask + (int64_t)t * mask_words;
   for (int w = threadIdx.x; w < mask_words; w += blockDim.x) mk[w] = 0u;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+  for (int x = threadIdx.x; x < nb + nbk; x += blockDim.x) {
+    const int side = x >= nb, b = side ? x - nb : x;
+    if (b >= kMaskBlocks) continue;
+    int* at = s_at[side][b];
     int cnt = 0;
     for (int k = 0; k < 64 && cnt <= kMaskAtoms; ++k) {
-      const int ao = am[b * 64 + k];
+      const int c = side ? ks[b * 64 + k] : b * 64 + k;
+      const int ao = c >= 0 ? am[c] : -1;
       if (ao < 0) continue;
       const int a = ao_atom[ao];
       bool seen = false;
-      for (int i = 0; i < cnt && i < kMaskAtoms; ++i) seen |= s_at[b][1 + i] == a;
+      for (int i = 0; i < cnt && i < kMaskAtoms; ++i) seen |= at[1 + i] == a;
       if (!seen) {
-        if (cnt < kMaskAtoms) s_at[b][1 + cnt] = a;
+        if (cnt < kMaskAtoms) at[1 + cnt] = a;
         ++cnt;
       }
     }
-    s_at[b][0] = cnt;
+    at[0] = cnt;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int bi = e / nb, bj = e % nb;  // nu block, mu block
-    bool on = bj == 0;
-    const int ci = s_at[bi][0], cj = s_at[bj][0];
+  for (int e = threadIdx.x; e < nb * nbk; e += blockDim.x) {
+    const int bi = e / nbk, bj = e % nbk;  // nu block, mu block
+    bool on = bj == 0 || bi >= kMaskBlocks || bj >= kMaskBlocks;
+    const int ci = on ? 0 : s_at[0][bi][0], cj = on ? 0 : s_at[1][bj][0];
     if (ci > kMaskAtoms || cj > kMaskAtoms) on = true;
     for (int i = 0; i < ci && !on; ++i)
-      for (int j = 0; j < cj && !on; ++j) on = nz[(int64_t)s_at[bi][1 + i] * natom + s_at[bj][1 + j]] != 0;
+      for (int j = 0; j < cj && !on; ++j) on = nz[(int64_t)s_at[0][bi][1 + i] * natom + s_at[1][bj][1 + j]] != 0;
     if (on) atomicOr(&mk[e >> 5], 1u << (e & 31));
   }
 }
@@ -401,7 +424,8 @@ __global__ void __launch_bounds__(256)
 struct TcArgs {
   TileBatch tb;
   int nqa;
-  const uint64_t* Dp;    // packed D digits (pack_digits5), Mpad x Mpad
+  const uint4* Dw;       // D digits 0-3, plane words per quad, Mpad x Mpad / 4
+  const uint32_t* Dlow;  // D digit 4
   const int32_t* fexp;   // D row exponents
   const int32_t* eexp;   // A row exponents [C][128]
   int Mpad;
@@ -521,14 +545,24 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   if (warp < 4) {
     // ---------------- producers
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kProducerRegs));
-    // Thread tid owns the 4 mu columns k4 = (tid % 16) * 4 of every stage and the
-    // 8 nu rows n = tid / 16 + 8 i of every nu tile; its 32 gathers of D are
-    // independent.  Stages are software-pipelined one ahead: the AO indices of
-    // stage j + 1 are requested before the wait for stage j's slot, and its
-    // gathers right after stage j's shared-memory writes, so the two dependent
-    // global latencies overlap the MMAs instead of adding up.
+    // Thread tid owns the quad tid % 16 of the stage's 16 quads of mu and the 8 nu
+    // rows tid / 16 + 8 i of every nu tile.  D is kept per row and quad as plane
+    // words, so a gather is one 16-byte and one 4-byte load and five 4-byte stores
+    // into the planes, with nothing in between; the K side of a tile therefore
+    // consists of whole quads (zero A digits where a quad's AO is not the tile's:
+    // 15 to 25% more columns with the AO order of ctc_basis.cu, 45% without).
+    //   The L1 bounds this role, next to the operand reads of the MMAs (864
+    // cycles of shared memory per stage): four 8-byte words per lane, transposed
+    // in registers, touch every sector of two rows with each of four loads (2.2 K
+    // cycles per stage); gathering lane = column coalesces the loads but needs a
+    // transpose through shared memory (3.2 K) or byte stores (14 K).
+    //   Stages are software-pipelined one ahead: the indices of stage j + 1 are
+    // requested before the wait for stage j's slot, and its gathers right after
+    // stage j's shared-memory writes, so the two dependent global latencies
+    // overlap the MMAs instead of adding up.
     const int tid = threadIdx.x;
-    const int k4 = (tid & 15) * 4, nrow0 = tid >> 4;
+    const int quad = tid & 15, nrow0 = tid >> 4;
+    const int qld = args.Mpad / 4;
     const uint64_t keep = policy_evict_last();
     int it = 0;  // stage counter across tiles
     // thread 0: stage counter of the last TMA issue into each slot (-1: none)
@@ -553,33 +587,34 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       if (item < 0 || warp_abort()) break;
       const int t = item / parts, part = item % parts;
       const int kt = tb.kt[t];
-      const int nkb = kt / kBK;
+      const int nkb = tb.kp[t] / kBK;
       const int nnt = (kt + kN - 1) / kN;
       const int nst = nnt > part ? (nnt - part + parts - 1) / parts * nkb : 0;  // of this part
       const int32_t* am = tb.aomap + (int64_t)t * tb.Kcap;
-      auto load_idx = [&](int j, int (&nu)[8], int (&mu)[4]) {
+      const int32_t* kq = tb.kq + (int64_t)t * (tb.Kpcap / 4);
+      auto load_idx = [&](int j, int (&nu)[8], int& mu) {
         const int n = j / nkb, kb = j - n * nkb, nt = part + n * parts;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int nc = nt * kN + nrow0 + 8 * q;
           nu[q] = am[nc < kt ? nc : 0];
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) mu[q] = am[kb * kBK + k4 + q];
+        mu = kq[kb * (kBK / 4) + quad];
       };
-      // Padding (-1) reads D's first row or column: the A digits of padding
-      // columns and the scales of padding rows are zero.  (A condition on the
-      // load makes the compiler wait for each one before the next: contraction
-      // of the 530 000-point cube 74.8 ms with it, 67.7 ms without.)
-      auto gather = [&](const int (&nu)[8], const int (&mu)[4], uint64_t (&w)[8][4]) {
+      // Padding rows (-1) read D's first row: their scales are zero.  (A condition
+      // on the load makes the compiler wait for each one before the next:
+      // contraction of the 530 000-point cube 74.8 ms with it, 67.7 ms without.)
+      auto gather = [&](const int (&nu)[8], int mu, uint4 (&w)[8], uint32_t (&lo)[8]) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-#pragma unroll
-          for (int m = 0; m < 4; ++m)
-            w[q][m] = ldg_u64_hint(args.Dp + (int64_t)max(nu[q], 0) * args.Mpad + max(mu[m], 0), keep);
+        for (int q = 0; q < 8; ++q) {
+          const int64_t o = (int64_t)max(nu[q], 0) * qld + mu;
+          w[q] = ldg_u128_hint(args.Dw + o, keep);
+          lo[q] = ldg_u32_hint(args.Dlow + o, keep);
+        }
       };
-      int nu[8], mu[4];
-      uint64_t w[8][4];
+      int nu[8], mu = 0;
+      uint4 w[8];
+      uint32_t lo[8];
       // the tile's active stages in order (every stage unless D is block-sparse)
       auto next_on = [&](int j) -> int {
         if (!sparse) return j;
@@ -589,7 +624,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       int j = next_on(0);
       if (j < nst) {
         load_idx(j, nu, mu);
-        gather(nu, mu, w);
+        gather(nu, mu, w, lo);
       }
       for (; j < nst; ++it) {
         const int jn = next_on(j + 1);
@@ -614,23 +649,16 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
         uint8_t* b = sB + s * kBStageBytes;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          // 4 words of 5 digit bytes -> 5 plane words of 4 consecutive mu:
-          // digits 0-3 by a byte transpose of the low halves, digit 4 from
-          // byte 4 of each word
-          uint32_t pl[4];
-          transpose_bytes4x4((uint32_t)w[q][0], (uint32_t)w[q][1], (uint32_t)w[q][2],
-                             (uint32_t)w[q][3], pl);
-          const uint32_t lo = __byte_perm(__byte_perm((uint32_t)(w[q][0] >> 32), (uint32_t)(w[q][1] >> 32), 0x0040),
-                                          __byte_perm((uint32_t)(w[q][2] >> 32), (uint32_t)(w[q][3] >> 32), 0x0040),
-                                          0x5410);
-          const uint32_t off = sw64_offset(nrow0 + 8 * q, k4);
-#pragma unroll
-          for (int p = 0; p < 4; ++p) *(uint32_t*)(b + p * kBPlaneBytes + off) = pl[p];
-          *(uint32_t*)(b + 4 * kBPlaneBytes + off) = lo;
+          uint8_t* o = b + sw64_offset(nrow0 + 8 * q, quad * 4);
+          *(uint32_t*)o = w[q].x;
+          *(uint32_t*)(o + kBPlaneBytes) = w[q].y;
+          *(uint32_t*)(o + 2 * kBPlaneBytes) = w[q].z;
+          *(uint32_t*)(o + 3 * kBPlaneBytes) = w[q].w;
+          *(uint32_t*)(o + 4 * kBPlaneBytes) = lo[q];
         }
         fence_proxy_async();
         mbar_arrive(&full_bar[s]);
-        if (more) gather(nu, mu, w);
+        if (more) gather(nu, mu, w, lo);
         j = jn;
       }
       if (warp_abort()) break;
@@ -668,7 +696,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       if (item < 0 || warp_abort()) break;
       const int t = item / parts;
       const int kt = tb.kt[t];
-      const int nkb = kt / kBK;
+      const int nkb = tb.kp[t] / kBK;
       const int nnt = (kt + kN - 1) / kN;
       bool failed = false;
       for (int nt = item % parts; nt < nnt && !failed; nt += parts, ++gnt) {
@@ -908,10 +936,10 @@ int prepare_tc(ctc_molecule* mol, cudaStream_t st) {
   CTC_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
   if (major != 10) return fail(CTC_ERR_UNSUPPORTED, "tensor-core split path needs an sm_100 GPU");
   const size_t MM = (size_t)mol->Mpad * mol->Mpad;
-  if (!mol->d_Dsl) CTC_CUDA_TRY(cudaMalloc((void**)&mol->d_Dsl, sizeof(uint64_t) * MM));
+  if (!mol->d_Dsl) CTC_CUDA_TRY(cudaMalloc((void**)&mol->d_Dsl, (size_t)kPlanes * MM));
   if (!mol->d_Dscale) CTC_CUDA_TRY(cudaMalloc((void**)&mol->d_Dscale, sizeof(int32_t) * mol->Mpad));
-  slice_d_kernel<<<mol->Mpad, 256, 0, st>>>(mol->d_D, mol->Mpad, (uint64_t*)mol->d_Dsl,
-                                            (int32_t*)mol->d_Dscale);
+  slice_d_kernel<<<mol->Mpad, 256, 0, st>>>(mol->d_D, mol->Mpad, (uint4*)mol->d_Dsl,
+                                            (uint32_t*)(mol->d_Dsl + 4 * MM), (int32_t*)mol->d_Dscale);
   CTC_CUDA_TRY(cudaGetLastError());
   // atom-pair map of D's non-zero blocks, kept only if some block is zero
   // (every AO on an atom, at most 4096 atoms: a map of 16 MB at most)
@@ -943,7 +971,7 @@ int prepare_tc(ctc_molecule* mol, cudaStream_t st) {
 // Chunk workspace of the tensor-core path, one layout for both users (the AO
 // kernel that writes the digit planes and the contraction), for tiles of
 // `rows` operand rows (ctc_split.cuh):
-//   planes [C][rows / 128][5][128][Kcap] int8 | eexp [C][rows] | stage masks
+//   planes [C][rows / 128][5][128][Kpcap] int8 | eexp [C][rows] | stage masks
 struct TcWorkspace {
   int8_t* planes;
   int32_t* eexp;
@@ -960,10 +988,9 @@ int tc_workspace(ctc_molecule* mol, const TileBatch& tb, int rows, cudaStream_t 
     off = (off + bytes + 255) / 256 * 256;
     return o;
   };
-  const size_t o_planes = take((size_t)tb.C * kPlanesA * rows * tb.Kcap);
+  const size_t o_planes = take((size_t)tb.C * kPlanesA * rows * tb.Kpcap);
   const size_t o_eexp = take(sizeof(int32_t) * (size_t)tb.C * rows);
-  const int nbmax = tb.Kcap / kBK;
-  const int mask_words = mol->d_nzpair ? (nbmax * nbmax + 31) / 32 : 0;
+  const int mask_words = mol->d_nzpair ? ((tb.Kcap / kN) * (tb.Kpcap / kBK) + 31) / 32 : 0;
   const size_t o_mask = take(sizeof(uint32_t) * (size_t)tb.C * mask_words);
   const size_t o_psum = take(sizeof(double) * 512 * (size_t)tb.C * std::min(kMaxParts, tb.Kcap / kN));
   int rc = mol->ws_sl.ensure(off, st);
@@ -1002,13 +1029,13 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   const int rows = split_tile_rows(tb.TP, plan.nqa);
   TcWorkspace w;
   if ((rc = tc_workspace(mol, tb, rows, st, &w)) != CTC_OK) return rc;
-  // tensor map over the planes: 2-D, rows = C * rows * 5, inner = Kcap bytes;
+  // tensor map over the planes: 2-D, rows = C * rows * 5, inner = Kpcap bytes;
   // boxes of 64 bytes (64-byte swizzle) by 128 rows
   PFN_cuTensorMapEncodeTiled_v12000 enc = get_encode();
   if (!enc) return fail(CTC_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
   CUtensorMap amap;
-  cuuint64_t gdim[2] = {(cuuint64_t)tb.Kcap, (cuuint64_t)tb.C * kPlanesA * rows};
-  cuuint64_t gstride[1] = {(cuuint64_t)tb.Kcap};
+  cuuint64_t gdim[2] = {(cuuint64_t)tb.Kpcap, (cuuint64_t)tb.C * kPlanesA * rows};
+  cuuint64_t gstride[1] = {(cuuint64_t)tb.Kpcap};
   cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kRows};
   cuuint32_t estr[2] = {1, 1};
   CUresult cr = enc(&amap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, w.planes, gdim, gstride, box, estr,
@@ -1021,7 +1048,8 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   TcArgs a;
   a.tb = tb;
   a.nqa = plan.nqa;
-  a.Dp = (const uint64_t*)mol->d_Dsl;
+  a.Dw = (const uint4*)mol->d_Dsl;
+  a.Dlow = (const uint32_t*)(mol->d_Dsl + 4 * (size_t)mol->Mpad * mol->Mpad);
   a.fexp = (const int32_t*)mol->d_Dscale;
   a.eexp = w.eexp;
   a.Mpad = mol->Mpad;
@@ -1061,9 +1089,10 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
   }
   if (trace_on) {
     std::vector<long long> tr((size_t)8 * grid);
-    std::vector<int32_t> kt(tb.C);
+    std::vector<int32_t> kt(tb.C), kp(tb.C);
     CTC_CUDA_TRY(cudaMemcpyAsync(tr.data(), a.trace, sizeof(long long) * tr.size(), cudaMemcpyDeviceToHost, st));
     CTC_CUDA_TRY(cudaMemcpyAsync(kt.data(), tb.kt, sizeof(int32_t) * tb.C, cudaMemcpyDeviceToHost, st));
+    CTC_CUDA_TRY(cudaMemcpyAsync(kp.data(), tb.kp, sizeof(int32_t) * tb.C, cudaMemcpyDeviceToHost, st));
     CTC_CUDA_TRY(cudaStreamSynchronize(st));
     CTC_CUDA_TRY(cudaFreeAsync(a.trace, st));
     double sum[8] = {0}, stages = 0, ktmax = 0, ktsum = 0, totmax = 0;
@@ -1072,7 +1101,7 @@ int tc_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb
       totmax = std::max(totmax, (double)tr[(size_t)8 * i]);
     }
     for (int i = 0; i < tb.C; ++i) {
-      stages += (kt[i] / (double)kBK) * std::ceil(kt[i] / (double)kN);
+      stages += (kp[i] / (double)kBK) * std::ceil(kt[i] / (double)kN);
       ktsum += kt[i];
       ktmax = std::max(ktmax, (double)kt[i]);
     }

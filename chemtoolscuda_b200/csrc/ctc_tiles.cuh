@@ -285,25 +285,39 @@ __device__ __forceinline__ bool seg_significant(const DevSeg& sg, const double* 
 constexpr int32_t kStatusCapacity = 0x7201;
 
 // Capacity pre-pass: the largest padded compact AO count of a batch of tiles
-// (atomicMax into *kmax).  One block per tile.
+// (atomicMax into kmax[0]) and a bound of the AOs in their quads (kmax[1]: each
+// run of consecutive AOs adds at most three at either end).  One block per tile.
 __global__ void __launch_bounds__(kTileThreads)
     tile_capacity_kernel(const DevSeg* __restrict__ segs, int nseg, TileBatch tb, int* kmax) {
   __shared__ double sctr[3], srad;
-  __shared__ int part[kTileThreads / 32];
+  __shared__ int part[2][kTileThreads / 32];
   const int t = blockIdx.x;
   tile_sphere(tb.xyz + (int64_t)t * tb.TP * 3, tb.TP, sctr, &srad);
-  int cnt = 0;
+  int cnt = 0, runs = 0;
   for (int s = threadIdx.x; s < nseg; s += kTileThreads) {
     const DevSeg sg = segs[s];
-    if (seg_significant(sg, sctr, srad)) cnt += ncomp_of_type_dev(sg.type);
+    if (seg_significant(sg, sctr, srad)) {
+      cnt += ncomp_of_type_dev(sg.type);
+      runs += s == 0 || !seg_significant(segs[s - 1], sctr, srad);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = cnt;
+  for (int o = 16; o > 0; o >>= 1) {
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    runs += __shfl_xor_sync(0xffffffffu, runs, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = cnt;
+    part[1][threadIdx.x >> 5] = runs;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int tot = 0;
-    for (int w = 0; w < kTileThreads / 32; ++w) tot += part[w];
+    int tot = 0, nr = 0;
+    for (int w = 0; w < kTileThreads / 32; ++w) {
+      tot += part[0][w];
+      nr += part[1][w];
+    }
     atomicMax(kmax, (tot + kKtAlign - 1) / kKtAlign * kKtAlign);
+    atomicMax(kmax + 1, (tot + 6 * nr + kKtAlign - 1) / kKtAlign * kKtAlign);
   }
 }
 
@@ -402,6 +416,40 @@ __global__ void __launch_bounds__(kTileThreads)
   const int kt_true = min(base_k, s_over_k);
   const int kt = min((kt_true + kKtAlign - 1) / kKtAlign * kKtAlign, tb.Kcap);
   for (int k = kt_true + threadIdx.x; k < kt; k += kTileThreads) am[k] = -1;
+  if (tb.Kpcap > 0) {
+    // quads of the compact AOs (ascending, as the AOs are) and the compact index
+    // of every place in them
+    int32_t* kq = tb.kq + (int64_t)t * (tb.Kpcap / 4);
+    int4* ks = reinterpret_cast<int4*>(tb.ksrc + (int64_t)t * tb.Kpcap);
+    const int qcap = tb.Kpcap / 4;
+    __syncthreads();
+    int nq = 0;
+    for (int k0 = 0; k0 < kt_true; k0 += kTileThreads) {
+      const int k = k0 + threadIdx.x;
+      const int ao = k < kt_true ? am[k] : 0;
+      const int first = k < kt_true && (k == 0 || (am[k - 1] >> 2) != (ao >> 2));
+      int before, total;
+      Scan(scan_tmp).ExclusiveSum(first, before, total);
+      const int q = nq + before + first - 1;
+      if (first && q < qcap) {
+        kq[q] = ao >> 2;
+        ks[q] = make_int4(-1, -1, -1, -1);
+      }
+      __syncthreads();
+      if (k < kt_true) {
+        if (q < qcap) tb.ksrc[(int64_t)t * tb.Kpcap + 4 * q + (ao & 3)] = k;
+        else atomicExch(status, kStatusCapacity);  // never, as above
+      }
+      nq += total;
+    }
+    nq = min(nq, qcap);
+    const int kp = (4 * nq + kKtAlign - 1) / kKtAlign * kKtAlign;
+    for (int q = nq + threadIdx.x; q < kp / 4; q += kTileThreads) {
+      kq[q] = 0;
+      ks[q] = make_int4(-1, -1, -1, -1);
+    }
+    if (threadIdx.x == 0) tb.kp[t] = kp;
+  }
   if (threadIdx.x == 0) {
     tb.nsig[t] = ns;
     tb.ktrue[t] = kt_true;
@@ -482,7 +530,7 @@ struct Carve {
   }
 };
 
-size_t tile_bytes(const ctc_molecule* mol, int C, int TP, int Kcap_) {
+size_t tile_bytes(const ctc_molecule* mol, int C, int TP, int Kcap_, int Kpcap = 0) {
   const size_t Kcap = Kcap_;
   size_t b = 0;
   auto add = [&](size_t x) { b = (b + 255) / 256 * 256 + x; };
@@ -496,17 +544,21 @@ size_t tile_bytes(const ctc_molecule* mol, int C, int TP, int Kcap_) {
   add(sizeof(int32_t) * (size_t)C * Kcap);
   add(sizeof(int32_t) * C);
   add(2 * sizeof(int32_t));
+  add(sizeof(int32_t) * C);
+  add(sizeof(int32_t) * (size_t)C * (Kpcap / 4));
+  add(sizeof(int32_t) * (size_t)C * Kpcap);
   return b + 256;
 }
 
 
 // Tile builder + chunk loop.  For every chunk: tile points, screen, AO block
 // (derivative order deriv, nq quantities; ao_launch replaces the plain AO
-// kernel launch when given), then compute(tb).
+// kernel launch when given), then compute(tb).  quads: the tensor-core
+// contraction's K side is formed too.
 inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, int nq, int deriv,
                      cudaStream_t st, const std::function<int(const TileBatch&)>& compute,
                      const std::function<int(const TileBatch&)>* ao_launch = nullptr,
-                     int rows = 128) {
+                     int rows = 128, bool quads = false) {
   if (n <= 0) return CTC_OK;  // (no zero-sized grids below)
   // cubic-grid tiles: blocks of 2x4x4 or 4x4x8 grid points
   int TX = 2, TY = 4, TZ = 4;
@@ -619,7 +671,7 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   // count-only screening pass over every tile of the call finds the largest
   // compact set and the workspace is sized for that instead.  It waits for
   // the stream once (to read the count back); smaller bases skip it.
-  int Kcap = mol->Mpad;
+  int Kcap = mol->Mpad, Kpcap = quads ? mol->Mpad : 0;
   if ((int64_t)(budget / (sizeof(double) * (size_t)nq * TP * mol->Mpad)) < 4 * 148 && ntiles > 148) {
     const int64_t PB = std::min<int64_t>(ntiles, 16384);
     const size_t pb_bytes = sizeof(double) * (size_t)PB * TP * 3 + sizeof(int64_t) * (size_t)PB * TP + 1024;
@@ -627,10 +679,10 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     TileBatch pb;
     pb.TP = TP;
     Carve cv{(char*)mol->ws_cap.p};
-    int* d_kmax = cv.take<int>(1);
+    int* d_kmax = cv.take<int>(2);
     pb.xyz = cv.take<double>((size_t)PB * TP * 3);
     pb.out = cv.take<int64_t>((size_t)PB * TP);
-    CTC_CUDA_TRY(cudaMemsetAsync(d_kmax, 0, sizeof(int), st));
+    CTC_CUDA_TRY(cudaMemsetAsync(d_kmax, 0, 2 * sizeof(int), st));
     for (int64_t t0 = 0; t0 < ntiles; t0 += PB) {
       pb.C = (int)std::min<int64_t>(PB, ntiles - t0);
       if ((rc = tile_points(pb, t0)) != CTC_OK) return rc;
@@ -638,9 +690,10 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
       CTC_CUDA_TRY(cudaGetLastError());
       mol->host_launches += 2;
     }
-    CTC_CUDA_TRY(cudaMemcpyAsync(mol->h_status + 1, d_kmax, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CTC_CUDA_TRY(cudaMemcpyAsync(mol->h_status + 1, d_kmax, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CTC_CUDA_TRY(cudaStreamSynchronize(st));
     Kcap = std::min(mol->Mpad, std::max(kKtAlign, (int)mol->h_status[1]));
+    if (quads) Kpcap = std::min(mol->Mpad, std::max(kKtAlign, (int)mol->h_status[2]));
   }
   const size_t ao_per_tile = sizeof(double) * (size_t)nq * TP * Kcap;
   int64_t C = 0;
@@ -651,7 +704,7 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     ask();  // a small block did not fit: the chunk that the free memory allows
   }
   if (rc != CTC_OK) return rc;
-  if ((rc = mol->ws_misc.ensure(tile_bytes(mol, (int)C, TP, Kcap), st)) != CTC_OK) return rc;
+  if ((rc = mol->ws_misc.ensure(tile_bytes(mol, (int)C, TP, Kcap, Kpcap), st)) != CTC_OK) return rc;
   int nsm = 148;
   if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   TileBatch tb;
@@ -672,6 +725,10 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     tb.order = cv.take<int32_t>(C);
     tb.counter = cv.take<int32_t>(2);
     tb.parts = tb.counter + 1;
+    tb.kp = cv.take<int32_t>(C);
+    tb.kq = cv.take<int32_t>((size_t)C * (Kpcap / 4));
+    tb.ksrc = cv.take<int32_t>((size_t)C * Kpcap);
+    tb.Kpcap = Kpcap;
   }
   for (int64_t t0 = 0; t0 < ntiles; t0 += C) {
     tb.C = (int)std::min<int64_t>(C, ntiles - t0);
