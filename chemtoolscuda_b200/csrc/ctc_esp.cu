@@ -403,7 +403,7 @@ __device__ __forceinline__ void esp_far_pair(const double4 q, const double2* __r
 // classes: row y of part.  Rows are summed in a fixed order by
 // esp_finish_kernel, so results do not depend on timing.
 // Bound: FP64 pipe (73% busy).  100 atoms (1 604 functions, 8e5 pairs), 1e5
-// surface points: far 110 ms and near 40 ms; one kernel per class with the R
+// surface points: far 110 ms and near 26 ms; one kernel per class with the R
 // recursion for every pair took 287 ms.
 template <int P>
 __global__ void __launch_bounds__(kEspThreads)
@@ -982,16 +982,19 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
     const int64_t gx = (m + P * kEspThreads - 1) / (P * kEspThreads);
     // slices of the batches: about 32 blocks per SM, at least a batch each
     const int64_t want = (32 * (int64_t)nsm + gx - 1) / gx;
-    const int S = e->nbatch == 0 ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)e->nbatch, 65535}));
+    const int S = e->nbatch == 0 ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)e->nbatch, 16383}));
+    // near pairs cluster in few batches: four times as many slices for them (near
+    // kernel at 1e5 surface points of 100 atoms: 40 -> 26 ms)
+    const int SN = std::min(4 * S, e->nbatch);
     const bool sort = m > kEspThreads;
     size_t tmp_bytes = 0;
     if (sort)
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                                    (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, kMortonSortBits, st));
-    const size_t need = sizeof(double) * (size_t)(2 * S + 3) * m + 4 * sizeof(int32_t) * (size_t)m + tmp_bytes + 4096;
+    const size_t need = sizeof(double) * (size_t)(S + SN + 3) * m + 4 * sizeof(int32_t) * (size_t)m + tmp_bytes + 4096;
     if (int rc = mol->ws_esp.ensure(need, st); rc != CTC_OK) return rc;
     Carve cv{(char*)mol->ws_esp.p};
-    double* part = cv.take<double>((size_t)std::max(1, 2 * S) * m);
+    double* part = cv.take<double>((size_t)std::max(1, S + SN) * m);
     double* xyz = cv.take<double>(3 * (size_t)m);
     int32_t* perm = nullptr;
     const unsigned g = (unsigned)((m + 255) / 256);
@@ -1011,16 +1014,16 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
     esp_gather_kernel<<<g, 256, 0, st>>>(pts, perm, m, xyz);
     CTC_CUDA_TRY(cudaGetLastError());
     if (S > 0) {
-      const dim3 grid((unsigned)gx, (unsigned)S);
+      const dim3 grid((unsigned)gx, (unsigned)S), ngrid((unsigned)gx, (unsigned)SN);
       double* near = part + (int64_t)S * m;
       if (P == 2) esp_far_kernel<2><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_far, e->d_batches, e->nbatch, xyz, m, part);
       else esp_far_kernel<1><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_far, e->d_batches, e->nbatch, xyz, m, part);
       CTC_CUDA_TRY(cudaGetLastError());
-      if (P == 2) esp_near_kernel<2><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
-      else esp_near_kernel<1><<<grid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
+      if (P == 2) esp_near_kernel<2><<<ngrid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
+      else esp_near_kernel<1><<<ngrid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
       CTC_CUDA_TRY(cudaGetLastError());
     }
-    esp_finish_kernel<<<g, 256, 0, st>>>(part, 2 * S, e->d_atoms, e->natom, xyz, perm, m, d_out + p0);
+    esp_finish_kernel<<<g, 256, 0, st>>>(part, S + SN, e->d_atoms, e->natom, xyz, perm, m, d_out + p0);
     CTC_CUDA_TRY(cudaGetLastError());
   }
   return CTC_OK;
