@@ -104,7 +104,8 @@ __device__ __forceinline__ void eval_dispatch(const DevSeg& sg, const double* __
 // row of the chunk is written as one run of consecutive addresses.  (One thread
 // per segment and point, stores M doubles apart and the terms read from
 // constant memory, took 990 us for values and gradients of 820 functions at
-// 30 000 points, 0.8 TB/s; this form 328 us.)
+// 30 000 points, 0.8 TB/s; this form 328 us, 420 with 32
+// AOs per chunk.)
 constexpr int kAoPubThreads = 256;
 __host__ __device__ constexpr int ao_chunk(int deriv) { return deriv == 2 ? 32 : 64; }
 __host__ __device__ constexpr size_t ao_pub_smem(int deriv) {
@@ -158,6 +159,8 @@ __global__ void __launch_bounds__(kAoPubThreads)
 // maximum of its values while it evaluates, so the exponents cost no second
 // pass over the block; slice_rows_kernel then writes the digit planes.
 //
+// With SLICE = 0 a tile's segments may be dealt out to gridDim.y CTAs.
+//
 // SLICE = -1 or -2 is the adjoint's form: from the weights of the tile's points
 // (dL/drho, dL/dgrad rho at their original index) it also writes the row
 // w = v_rho phi + v_grad . grad phi, as quantity 10 behind the ten AO quantities
@@ -193,7 +196,7 @@ __global__ void __launch_bounds__(kAoThreads, 3)
         for (int k = 0; k < 3; ++k) wv[1 + k] = v_grad[3 * oi + k];
       }
     }
-    for (int i = warp; i < ns; i += kAoThreads / 32) {
+    for (int i = warp + blockIdx.y * (kAoThreads / 32); i < ns; i += gridDim.y * (kAoThreads / 32)) {
       const DevSeg sg = segs[sl[i]];
       eval_dispatch<DERIV, SLICE>(sg, alpha, coef, px, py, pz, A + (int64_t)k0[i] * TP + j, ld_q, TP,
                                   tb.nq, mx, wv);
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kAoThreads, 3)
   }
   const int kt_true = tb.ktrue[t], kt = tb.kt[t];
   const int npad = (kt - kt_true) * TP;
-  for (int idx = threadIdx.x; idx < tb.nq * npad; idx += kAoThreads) {
+  for (int idx = threadIdx.x; idx < tb.nq * npad && blockIdx.y == 0; idx += kAoThreads) {
     const int q = idx / npad, r = idx % npad;
     A[q * ld_q + (int64_t)kt_true * TP + r] = 0.0;
   }
@@ -275,10 +278,13 @@ int launch_ao_tiles(const ctc_molecule* mol, const TileBatch& tb, int deriv, cud
   if (tb.C <= 0) return CTC_OK;
   const auto* sg = mol->d_segs;
   const double *al = mol->d_alpha, *co = mol->d_coef;
+  // few tiles: their segments on more CTAs, up to three for every SM (values of
+  // 62 segments at 200 points, seven tiles: 18 us on one CTA each, 5.5 on eight)
+  const dim3 grid((unsigned)tb.C, (unsigned)std::max(1, std::min(8, 3 * 148 / tb.C)));
   switch (deriv) {
-    case 0: ao_tile_kernel<0, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
-    case 1: ao_tile_kernel<1, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
-    default: ao_tile_kernel<2, 0><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr);
+    case 0: ao_tile_kernel<0, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
+    case 1: ao_tile_kernel<1, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
+    default: ao_tile_kernel<2, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr);
   }
   CTC_CUDA_TRY(cudaGetLastError());
   return CTC_OK;
