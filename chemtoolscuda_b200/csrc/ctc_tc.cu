@@ -283,12 +283,13 @@ __device__ __forceinline__ void contract_role(const double* __restrict__ ao, int
 // One nu tile of the contraction for NQA = 1 (rows are the tile's 128
 // points; thread etid owns point etid): acc[q] += sum_nu G[nu][etid] A_q[nu]
 // for the NQ AO quantities, the columns in order.  The AO values stream in
-// groups of GW columns through 4 register buffers (3 groups in flight).
+// groups of GW columns through NB register buffers (NB - 1 groups in flight): as
+// many as the epilogue's registers hold, as the loads are latency-bound.
 template <int NQ, int GW>
 __device__ __forceinline__ void contract_rows(const double* __restrict__ ao, int64_t ldq,
                                               const double* __restrict__ sG, int etid, uint64_t stream,
                                               double* acc) {
-  constexpr int NB = 4;
+  constexpr int NB = NQ == 4 ? 10 : 12;
   constexpr int NG = kN / GW;
   double a[NB][NQ][GW];
   auto load = [&](int buf, int cg) {
