@@ -24,8 +24,8 @@
 // tile's nu slices dealt out to up to eight of them, tiles largest first -- from
 // a launch-wide counter): warps 0-3 produce the
 // operands of each K block (one thread issues the TMA loads of the five A
-// planes; all 128 threads gather the five D planes by compact index from the
-// packed copy of D and write them in the 64-byte-swizzled K-major layout),
+// planes; all 128 threads gather D's plane words by nu row and quad of mu and
+// write them in the 64-byte-swizzled K-major layout),
 // warps 4-7 drain the TMEM accumulators (one 32-lane quarter each) into an
 // FP64 copy of G in shared memory and run the epilogue while the next nu
 // tile's MMAs run, warp 8 issues the MMAs from one thread and commits them to

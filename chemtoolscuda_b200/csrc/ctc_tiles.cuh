@@ -703,6 +703,7 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   int64_t C = 0;
   for (;;) {
     C = std::min<int64_t>(std::max<int64_t>(148, (int64_t)(budget / ao_per_tile)), ntiles);
+    if (C < ntiles) C -= C % 148;  // whole rounds of one tile per SM
     rc = mol->ws_ao.ensure(ao_per_tile * C, st);
     if (rc != CTC_ERR_NOMEM || asked) break;
     ask();  // a small block did not fit: the chunk that the free memory allows
