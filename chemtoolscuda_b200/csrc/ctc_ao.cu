@@ -278,9 +278,10 @@ int launch_ao_tiles(const ctc_molecule* mol, const TileBatch& tb, int deriv, cud
   if (tb.C <= 0) return CTC_OK;
   const auto* sg = mol->d_segs;
   const double *al = mol->d_alpha, *co = mol->d_coef;
-  // few tiles: their segments on more CTAs, up to three for every SM (values of
+  // few tiles: their segments on more CTAs, up to twelve for every SM, of which
+  // three or more run at a time, so that the last round is a small part (values of
   // 62 segments at 200 points, seven tiles: 18 us on one CTA each, 5.5 on eight)
-  const dim3 grid((unsigned)tb.C, (unsigned)std::max(1, std::min(8, 3 * 148 / tb.C)));
+  const dim3 grid((unsigned)tb.C, (unsigned)std::max(1, std::min(8, (12 * 148 + tb.C - 1) / tb.C)));
   switch (deriv) {
     case 0: ao_tile_kernel<0, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
     case 1: ao_tile_kernel<1, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;

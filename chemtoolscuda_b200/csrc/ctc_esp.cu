@@ -1006,7 +1006,7 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
       void* tmp = cv.take<char>(tmp_bytes);
       double lo[3], ext = 0;
       morton_box(mol, lo, &ext);
-      morton_kernel<<<g, 256, 0, st>>>(pts, m, lo[0], lo[1], lo[2], 1024.0 / ext, k_in, v_in);
+      morton_kernel<<<g, 256, 0, st>>>(pts, m, lo[0], lo[1], lo[2], kMortonCells / ext, k_in, v_in);
       CTC_CUDA_TRY(cudaGetLastError());
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k_in, k_out, v_in, perm, (int)m, 0,
                                                    kMortonSortBits, st));

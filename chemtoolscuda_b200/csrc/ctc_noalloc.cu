@@ -154,7 +154,7 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
   }
 
   morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_points, n, lo[0], lo[1], lo[2],
-                                                              1024.0 / ext, k_in, v_in);
+                                                              kMortonCells / ext, k_in, v_in);
   CTC_CUDA_TRY(cudaGetLastError());
   CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, sort_tmp, k_in, k_out, v_in, perm, (int)n, 0,
                                                kMortonSortBits, st));

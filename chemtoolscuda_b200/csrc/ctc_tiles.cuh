@@ -51,13 +51,16 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   return v;
 }
 
-// 30-bit Morton key of each point (the single-sort order of small calls and
+// 24-bit Morton key of each point (the single-sort order of small calls and
 // of the fixed-scratch entry point, ctc_noalloc.cu); a point with a
 // non-finite coordinate gets
-// kNonFiniteKey, so the sort puts such points after every finite one and they
-// share tiles only with each other (and at most one tile's finite points).
-constexpr uint32_t kNonFiniteKey = 1u << 30;
-constexpr int kMortonSortBits = 31;
+// kNonFiniteKey, the last one, so the sort puts such points behind the others
+// (but for points in the box's last cell).  Cells of 1/256 of the box (0.14 bohr
+// for 12 atoms) are well below a tile's size for the calls that use this order,
+// and 24 bits take three passes of the radix sort instead of four.
+constexpr uint32_t kNonFiniteKey = (1u << 24) - 1u;
+constexpr int kMortonCells = 256;
+constexpr int kMortonSortBits = 24;
 
 __global__ void morton_kernel(const double* __restrict__ pts, int64_t n, double lox, double loy,
                               double loz, double inv_cell, uint32_t* keys, int32_t* vals) {
@@ -65,7 +68,7 @@ __global__ void morton_kernel(const double* __restrict__ pts, int64_t n, double 
   if (i >= n) return;
   auto q = [&](double v, double lo) {
     double c = (v - lo) * inv_cell;
-    c = c < 0.0 ? 0.0 : (c > 1023.0 ? 1023.0 : c);
+    c = c < 0.0 ? 0.0 : (c > kMortonCells - 1.0 ? kMortonCells - 1.0 : c);
     return (uint32_t)c;
   };
   const double x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
@@ -577,7 +580,7 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   }
   int rc;
   // explicit points: sort-tile-recursive order over the points' own box for
-  // calls of kStrMinPoints points or more; below that, one sort of 30-bit
+  // calls of kStrMinPoints points or more; below that, one sort of 24-bit
   // Morton keys over the molecule's box padded by 12 bohr (three sorts cost
   // ~0.4 ms, as much as a whole 1e5-point density call of a small molecule,
   // while the tiles' shape matters little there)
@@ -623,7 +626,7 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
       morton_box(mol, lo, &ext);
       uint32_t* k32_in = (uint32_t*)k_in;
       uint32_t* k32_out = (uint32_t*)k_out;
-      morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src.pts, n, lo[0], lo[1], lo[2], 1024.0 / ext,
+      morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src.pts, n, lo[0], lo[1], lo[2], kMortonCells / ext,
                                                                   k32_in, v_in);
       CTC_CUDA_TRY(cudaGetLastError());
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k32_in, k32_out, v_in, perm, (int)n, 0,
