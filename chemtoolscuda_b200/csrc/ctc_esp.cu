@@ -991,19 +991,29 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
     if (sort)
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                                    (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, kMortonSortBits, st));
-    const size_t need = sizeof(double) * (size_t)(S + SN + 3) * m + 4 * sizeof(int32_t) * (size_t)m + tmp_bytes + 4096;
-    if (int rc = mol->ws_esp.ensure(need, st); rc != CTC_OK) return rc;
-    Carve cv{(char*)mol->ws_esp.p};
-    double* part = cv.take<double>((size_t)std::max(1, S + SN) * m);
-    double* xyz = cv.take<double>(3 * (size_t)m);
-    int32_t* perm = nullptr;
+    // One layout gives both the size of the block and the places in it (S and SN
+    // are zero when no pair is kept; the finish kernel then reads no row).
+    double *part = nullptr, *xyz = nullptr;
+    uint32_t *k_in = nullptr, *k_out = nullptr;
+    int32_t *v_in = nullptr, *perm = nullptr;
+    void* tmp = nullptr;
+    auto lay_out = [&](char* base) {
+      Carve cv{base};
+      part = cv.take<double>((size_t)(S + SN) * m);
+      xyz = cv.take<double>(3 * (size_t)m);
+      if (sort) {
+        k_in = cv.take<uint32_t>(m);
+        k_out = cv.take<uint32_t>(m);
+        v_in = cv.take<int32_t>(m);
+        perm = cv.take<int32_t>(m);
+        tmp = cv.take<char>(tmp_bytes);
+      }
+      return cv.off;
+    };
+    if (int rc = mol->ws_esp.ensure(lay_out(nullptr), st); rc != CTC_OK) return rc;
+    lay_out((char*)mol->ws_esp.p);
     const unsigned g = (unsigned)((m + 255) / 256);
     if (sort) {
-      uint32_t* k_in = cv.take<uint32_t>(m);
-      uint32_t* k_out = cv.take<uint32_t>(m);
-      int32_t* v_in = cv.take<int32_t>(m);
-      perm = cv.take<int32_t>(m);
-      void* tmp = cv.take<char>(tmp_bytes);
       double lo[3], ext = 0;
       morton_box(mol, lo, &ext);
       morton_kernel<<<g, 256, 0, st>>>(pts, m, lo[0], lo[1], lo[2], kMortonCells / ext, k_in, v_in);
