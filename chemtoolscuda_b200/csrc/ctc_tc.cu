@@ -469,7 +469,11 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __shared__ uint32_t tmem_base_sh;
   __shared__ int s_abort;
   __shared__ int s_tile[2];  // work item: tile * parts + part
-  __shared__ int s_epi_tile;
+  // the epilogue's work item, slot i & 1 for the CTA's i-th: a warp may still read
+  // slot i while etid 0 writes slot i + 1; slot i + 2 is written behind the barrier
+  // of item i + 1, which a warp reaches after it has read slot i (an item without
+  // slices has no other barrier)
+  __shared__ int s_epi_tile[2];
   __shared__ int s_epi_abort[2];
   __shared__ double s_cscale[2][kN];
 
@@ -782,11 +786,11 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
     for (int i = 0; !stop; ++i) {
       // one reader for the four warps keeps their decisions uniform
       if (etid == 0) {
-        s_epi_tile = read_tile(i);
+        s_epi_tile[i & 1] = read_tile(i);
         mbar_arrive(&tile_empty_bar[i & 1]);
       }
       asm volatile("bar.sync 1, 128;\n" ::: "memory");
-      const int item = s_epi_tile;
+      const int item = s_epi_tile[i & 1];
       if (item < 0) break;
       const int t = item / parts;
       const int kt = tb.kt[t];
