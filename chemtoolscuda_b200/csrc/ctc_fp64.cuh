@@ -32,8 +32,9 @@
 //   rho and gradient (full sums), 60 atoms, 268 800 points: 10.1 -> 7.1 ms
 //   dL/dR, same points: 60.8 -> 15.8 ms
 //
-// Every barrier wait is bounded: after the limit a role records
-// kStatusFp64Timeout, stops, and the CTA exits once its copies have landed.
+// Every barrier wait is bounded (ctc_molecule_set_wait_limit): after the limit a
+// role sets the CTA's abort flag and stops, the others' waits run out in turn, and
+// the CTA records kStatusFp64Timeout and exits once its copies have landed.
 #pragma once
 
 #include "ctc_internal.h"
@@ -59,6 +60,7 @@ static_assert(128 * kFProducerRegs + 128 * kFEpilogueRegs + 256 * kFMatrixRegs <
               "register split above the launch's total");
 static_assert(kKtAlign % kFN == 0 && kFN % kFK == 0, "tile K alignment");
 constexpr int32_t kStatusFp64Timeout = 0x7102;
+constexpr long long kLandCycles = 100000000LL;  // ~50 ms; a copy takes microseconds
 
 // What a launch computes.
 enum Fp64Mode {
@@ -234,6 +236,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
   __shared__ __align__(8) uint64_t full_bar[kFStages], tma_bar[kFStages], empty_bar[kFStages], gfull_bar, gempty_bar, gwide_bar;
   __shared__ double s_sums[32][kFSums + 1];
   __shared__ int s_abort, s_epi_abort;
+  __shared__ int s_issued[kFStages][2];  // stage counter of each half's last copies into a slot, -1: none
 
   const TileBatch& tb = args.tb;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
       mbar_init(&full_bar[s], 64);
       mbar_init(&tma_bar[s], 2);
       mbar_init(&empty_bar[s], 8);
+      s_issued[s][0] = s_issued[s][1] = -1;
     }
     mbar_init(&gfull_bar, 8);
     mbar_init(&gempty_bar, 4);
@@ -312,9 +316,6 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
 #pragma unroll
       for (int k = 0; k < kFK; ++k) v[k] = __ldg(d + (int64_t)__shfl_sync(0xffffffffu, m, k) * args.Mpad);
     };
-    int last_issue[kFStages];
-#pragma unroll
-    for (int s = 0; s < kFStages; ++s) last_issue[s] = -1;
     Cur cur{};
     open_tile(cur);
     if (pair) advance(cur);
@@ -341,31 +342,22 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
         const bool wide = !NARROW_ONLY && cur.kb < cur.wide;
         constexpr int NRUN = MODE == kFLocal4 ? 4 : (MODE == kFForce2 ? 2 : 1);  // quantities of a wide stage
         const int runs = wide ? NRUN : 1;
-        if (lane == 0) mbar_arrive_expect_tx(&tma_bar[s], 16 * runs * PTS * 8);
+        if (lane == 0) {
+          s_issued[s][khalf] = it;
+          mbar_arrive_expect_tx(&tma_bar[s], 16 * runs * PTS * 8);
+        }
         __syncwarp();
         for (int x = lane; x < 16 * runs; x += 32) {
           const int kk = 16 * khalf + x / runs, r = x % runs;
           const int q = MODE == kFForce2 ? 10 * r : r;
           bulk_copy(a + kk * kFALd + r * PTS, A + q * ldq + (int64_t)kk * PTS, PTS * 8, &tma_bar[s]);
         }
-#pragma unroll
-        for (int z = 0; z < kFStages; ++z)
-          if (z == s) last_issue[z] = it;
       }
 #pragma unroll
       for (int k = 0; k < kFK; ++k) b[k * kFBLd + ptid] = (nu_ok && ((ok >> k) & 1u)) ? v[k] : 0.0;
       mbar_arrive(&full_bar[s]);
       if (nxt.t >= 0) gather(mu, nu);
       cur = nxt;
-    }
-    // No copy may land after the CTA has left.  After a normal end the matrix
-    // warps wait for every one; after a timeout some may be on their way, and
-    // each slot's last copies are waited for with the full limit (a slot that the
-    // other pair has used since is past that phase: its wait runs out).
-    if (s_abort) {
-#pragma unroll
-      for (int s = 0; s < kFStages; ++s)
-        if (last_issue[s] >= 0) mbar_wait(&tma_bar[s], (last_issue[s] / kFStages) & 1);
     }
   } else if (warp >= 8) {
     // ---------------- matrix warps
@@ -649,7 +641,19 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
     }
   }
   __syncthreads();
-  if (s_abort && threadIdx.x == 0) atomicExch(args.status, kStatusFp64Timeout);
+  // No copy may land after the CTA has left.  After a normal end the matrix warps
+  // have waited for every one.  After a timeout in any role -- every warp is here,
+  // so s_abort is final and nothing is issued any more -- copies may be on their
+  // way, also those of producers that ended normally.  A slot's last stage is
+  // waited for with the full limit; where one of its two warps has not issued its
+  // half, the phase cannot end and kLandCycles gives the other half time to land.
+  if (s_abort && threadIdx.x == 0) {
+    for (int s = 0; s < kFStages; ++s) {
+      const int x = s_issued[s][0], y = s_issued[s][1], last = max(x, y);
+      if (last >= 0) mbar_wait(&tma_bar[s], (last / kFStages) & 1, x == y ? kWaitCycles : kLandCycles);
+    }
+    atomicExch(args.status, kStatusFp64Timeout);
+  }
 }
 
 // Launches one chunk; args holds what the mode needs beyond the tiles.
@@ -663,7 +667,7 @@ int launch_fp64(ctc_molecule* mol, const TileBatch& tb, Fp64Args args, cudaStrea
   args.Mpad = mol->Mpad;
   args.sym = mol->d_sym;
   args.status = mol->d_status;
-  args.wait_cycles = kWaitCycles;
+  args.wait_cycles = mol->wait_cycles > 0 ? (long long)mol->wait_cycles : kWaitCycles;
   fp64_tile_kernel<MODE><<<tb.C < nsm ? tb.C : nsm, kFThreads, kFSmem, st>>>(args);
   CTC_CUDA_TRY(cudaGetLastError());
   return CTC_OK;

@@ -185,7 +185,7 @@ struct ctc_molecule {
   int32_t* h_status = nullptr;
   cudaEvent_t status_ev = nullptr;
   bool status_pending = false;
-  // limit of the tensor-core pipeline's waits in SM cycles (0: the default)
+  // limit of the contraction pipelines' waits in SM cycles (0: the default)
   int64_t wait_cycles = 0;
   // work counters: [0] tiles [1] points [2] sum kt_true [3] sum rows*kt^2 (device, doubles)
   double* d_stats = nullptr;

@@ -268,11 +268,11 @@ int ctc_molecule_set_profiling(ctc_molecule* mol, int32_t on);
  * cudaError_t into a C++ exception (include/cuda_utils.cuh:55-60). */
 int ctc_molecule_sync_status(ctc_molecule* mol, void* stream);
 
-/* Limit, in SM clock cycles, of every wait in the tensor-core pipeline
- * (0 = the default of 4e9 cycles, about 2 s).  A kernel whose wait runs out
- * stops issuing work, waits for its own copies in flight, frees its tensor
- * memory, records CTC_ERR_DEVICE in the status word and returns; the
- * molecule stays usable.  A short limit makes the waits run out on purpose
+/* Limit, in SM clock cycles, of every wait in the pipelines of the tensor-core
+ * and the FP64 contraction (0 = the default of 4e9 cycles, about 2 s).  A
+ * kernel whose wait runs out stops issuing work, waits for its own copies in
+ * flight, frees its tensor memory, records CTC_ERR_DEVICE in the status word
+ * and returns; the molecule stays usable.  A short limit makes the waits run out on purpose
  * (tests of that path); no counterpart in the reference. */
 int ctc_molecule_set_wait_limit(ctc_molecule* mol, int64_t cycles);
 
