@@ -186,6 +186,8 @@ __global__ void upper_to_dldd_kernel(const double* __restrict__ Cacc, int M, int
 int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const double* v_rho,
                  const double* v_grad, double* dLdD, double* dLdR, cudaStream_t st) {
   if (n > (int64_t)INT32_MAX) return fail(CTC_ERR_INVALID, "adjoint: at most 2^31-1 points per call");
+  // a failure an earlier stream-ordered call recorded on the device
+  if (int rc = poll_status(mol, st); rc != CTC_OK) return rc;
   PointSrc src{};
   src.pts = d_points;
   // AO quantities: what the outputs asked for need and no more
@@ -239,7 +241,8 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
                                                                         mol->d_ao_iperm, dLdD);
     CTC_CUDA_TRY(cudaGetLastError());
   }
-  return CTC_OK;
+  // a wait of the force contraction that ran out, a tile beyond the workspace
+  return post_status(mol, st);
 }
 
 }  // namespace ctc

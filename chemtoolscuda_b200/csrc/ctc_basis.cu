@@ -183,11 +183,14 @@ void Scratch::release() {
 }
 
 // The status word.  Kernels that can fail on the device (bounded waits of the
-// tensor-core pipeline) set the molecule's device word with atomicExch; it
+// contraction pipelines) set the molecule's device word with atomicExch; it
 // stays set until it is reported.  After such kernels post_status enqueues a
 // copy of it into pinned host memory and records an event, so the call
 // itself never waits.  poll_status (at the start of the next call) reports a
-// copy that has landed; check_status waits for the stream first.
+// copy that has landed; check_status waits for the stream first.  While the
+// stream is being captured neither does anything (an event recorded in a capture
+// cannot be asked): a failure of the graph's kernels stays in the word until the
+// next call outside a capture has posted it, or until check_status.
 static std::string status_message(int32_t code) {
   if (code == 0x7101)
     return "a bounded wait of the tensor-core contraction ran out (status 0x7101); "
@@ -210,7 +213,17 @@ static int report_status(ctc_molecule* mol, cudaStream_t st, const char* what) {
   return fail(CTC_ERR_DEVICE, std::string(what) + ": " + status_message(h));
 }
 
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return c != cudaStreamCaptureStatusNone;
+}
+
 int post_status(ctc_molecule* mol, cudaStream_t st) {
+  if (capturing(st)) return CTC_OK;
   CTC_CUDA_TRY(cudaMemcpyAsync(mol->h_status, mol->d_status, sizeof(int32_t),
                                cudaMemcpyDeviceToHost, st));
   CTC_CUDA_TRY(cudaEventRecord(mol->status_ev, st));
@@ -219,7 +232,7 @@ int post_status(ctc_molecule* mol, cudaStream_t st) {
 }
 
 int poll_status(ctc_molecule* mol, cudaStream_t st) {
-  if (!mol->status_pending) return CTC_OK;
+  if (!mol->status_pending || capturing(st)) return CTC_OK;
   const cudaError_t q = cudaEventQuery(mol->status_ev);
   if (q == cudaErrorNotReady) return CTC_OK;
   CTC_CUDA_TRY(q);

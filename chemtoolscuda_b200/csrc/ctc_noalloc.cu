@@ -89,6 +89,8 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
   void* base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc != CTC_OK) return rc;
+  // a failure an earlier stream-ordered call recorded on the device
+  if ((rc = poll_status(mol, st)) != CTC_OK) return rc;
 
   const LocalPlan plan = plan_local(out);
   const int TP = fp64_tile_points(plan, n);
@@ -174,7 +176,7 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
     mol->host_launches += 5;
     mol->host_chunks += 1;
   }
-  return CTC_OK;
+  return post_status(mol, st);
 }
 
 }  // namespace

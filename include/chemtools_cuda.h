@@ -13,10 +13,11 @@
  * Device-pointer entry points are stream-ordered on the stream passed in
  * (NULL = legacy default stream) and return before the work finishes; they
  * do not synchronise.  A failure that a kernel detects on the device (a
- * bounded wait of the tensor-core pipeline running out) is recorded in the
- * molecule's status word and reported as CTC_ERR_DEVICE by the next call on
- * that molecule whose copy of the word has landed, or at once by
- * ctc_molecule_sync_status.  Use one stream at a time per molecule.  The
+ * bounded wait of a contraction's pipeline running out) is recorded in the
+ * molecule's status word and reported as CTC_ERR_DEVICE by the next
+ * descriptor or adjoint call on that molecule once the word's copy has landed,
+ * or at once by ctc_molecule_sync_status (which is also where a replayed
+ * graph's failure shows).  Use one stream at a time per molecule.  The
  * *_host variants take host pointers, copy inputs and outputs themselves and
  * return after the results are in host memory (and report device failures
  * of their own kernels).
