@@ -531,7 +531,10 @@ int ctc_molecule_create(const ctc_basis* b, int32_t natom, const double* atom_xy
       cudaMallocHost((void**)&m->h_status, 4 * sizeof(int32_t)) != cudaSuccess ||
       cudaEventCreateWithFlags(&m->status_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaMalloc((void**)&m->d_stats, sizeof(double) * 8) != cudaSuccess ||
-      cudaMemset(m->d_stats, 0, sizeof(double) * 8) != cudaSuccess) {
+      cudaMemset(m->d_stats, 0, sizeof(double) * 8) != cudaSuccess ||
+      // the memsets and the symmetry kernel are done when the molecule is handed
+      // out: a call on a non-blocking stream is not ordered behind them
+      cudaStreamSynchronize(0) != cudaSuccess) {
     ctc_molecule_destroy(m);
     return fail(CTC_ERR_NOMEM, "status word allocation failed");
   }
