@@ -18,6 +18,7 @@
 #include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 
+#include "ctc_chunk.h"
 #include "ctc_internal.h"
 #include "ctc_finalize.cuh"
 
@@ -647,14 +648,11 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   };
   // chunk of tiles: AO block (nq x TP x Kcap doubles per tile) within
   // min(12 GiB, a quarter of the free device memory) (CTC_CHUNK_BYTES
-  // overrides), at least one full wave of CTAs on 148 SMs.  Larger chunks
+  // overrides), at least one tile per SM (ctc_chunk.h).  Larger chunks
   // amortise the per-chunk launches and tails: on the 215^3 benchmark cube
   // 6 GiB gave 20.95 M points/s, 12 GiB 21.46 M, 24 GiB 21.60 M.
-  // The driver is asked for the free memory only when the answer can matter
-  // (the question takes 0.1 to 6 ms on a shared host, as long as a whole call
-  // of 1e5 points): not for calls whose blocks fit what the molecule already
-  // holds or 64 MiB, nor once it holds all that the limit allows.
-  constexpr size_t kMostAo = (size_t)12 << 30, kSmallAo = (size_t)64 << 20;
+  int nsm = 148;
+  if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   const size_t held = mol->ws_ao.bytes, tile_most = sizeof(double) * (size_t)nq * TP * mol->Mpad;
   size_t budget = kMostAo;
   bool asked = false;
@@ -671,7 +669,6 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
       asked = true;
     }
   }
-  if (!asked && tile_most * (size_t)ntiles > std::max(held, kSmallAo) && held + tile_most < kMostAo) ask();
   // Capacity of a tile's compact AO set: Mpad always suffices.  When a chunk
   // sized for Mpad columns would hold fewer than four waves of tiles (large
   // bases: the 1 000-atom molecule keeps ~350 of 16 128 functions per tile), a
@@ -679,7 +676,9 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   // compact set and the workspace is sized for that instead.  It waits for
   // the stream once (to read the count back); smaller bases skip it.
   int Kcap = mol->Mpad, Kpcap = quads ? mol->Mpad : 0;
-  if ((int64_t)(budget / (sizeof(double) * (size_t)nq * TP * mol->Mpad)) < 4 * 148 && ntiles > 148) {
+  auto few_tiles = [&]() { return (int64_t)(budget / tile_most) < 4 * nsm && ntiles > nsm; };
+  if (!asked && !few_tiles() && ask_free_memory(tile_most * chunk_tiles(budget, tile_most, ntiles, nsm), held)) ask();
+  if (few_tiles()) {
     const int64_t PB = std::min<int64_t>(ntiles, 16384);
     const size_t pb_bytes = sizeof(double) * (size_t)PB * TP * 3 + sizeof(int64_t) * (size_t)PB * TP + 1024;
     if ((rc = mol->ws_cap.ensure(pb_bytes, st)) != CTC_OK) return rc;
@@ -703,18 +702,19 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
     if (quads) Kpcap = std::min(mol->Mpad, std::max(kKtAlign, (int)mol->h_status[2]));
   }
   const size_t ao_per_tile = sizeof(double) * (size_t)nq * TP * Kcap;
-  int64_t C = 0;
-  for (;;) {
-    C = std::min<int64_t>(std::max<int64_t>(148, (int64_t)(budget / ao_per_tile)), ntiles);
-    if (C < ntiles) C -= C % 148;  // whole rounds of one tile per SM
-    rc = mol->ws_ao.ensure(ao_per_tile * C, st);
-    if (rc != CTC_ERR_NOMEM || asked) break;
+  int64_t C = chunk_tiles(budget, ao_per_tile, ntiles, nsm);
+  if (!asked && ask_free_memory(ao_per_tile * C, held)) {
+    ask();
+    C = chunk_tiles(budget, ao_per_tile, ntiles, nsm);
+  }
+  rc = mol->ws_ao.ensure(ao_per_tile * C, st);
+  if (rc == CTC_ERR_NOMEM && !asked) {
     ask();  // a small block did not fit: the chunk that the free memory allows
+    C = chunk_tiles(budget, ao_per_tile, ntiles, nsm);
+    rc = mol->ws_ao.ensure(ao_per_tile * C, st);
   }
   if (rc != CTC_OK) return rc;
   if ((rc = mol->ws_misc.ensure(tile_bytes(mol, (int)C, TP, Kcap, Kpcap), st)) != CTC_OK) return rc;
-  int nsm = 148;
-  if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   TileBatch tb;
   tb.TP = TP;
   tb.Kcap = Kcap;
