@@ -131,6 +131,7 @@ struct EspTables {
   EspBatch* d_batches = nullptr;
   double* d_atoms = nullptr;  // x y z Z per atom
   int npairs = 0, nbatch = 0, natom = 0;
+  bool s_only = false;        // every kept pair is of class 0
   size_t nh = 0;
   // algorithmic FP64 work per point: sum over the kept pairs of
   // 2 n_tuv(L) (contraction) + 2 n_R(L) (R recursion) + 10 (L + 1) (Boys)
@@ -252,10 +253,11 @@ __global__ void __launch_bounds__(256)
   for (int d = 0; d < 3; ++d) xyz[d * n + i] = pts[3 * p + d];
 }
 
-// A point as the pair sums see it: finite coordinates are cut at 1e100 bohr, so
-// that |P - C|^2 stays finite (the potential there is zero to any precision).
+// A point as the pair sums see it: finite coordinates are cut at 1e153 bohr, so
+// that |P - C|^2 stays finite (esp_finish_kernel gives zero beyond).
+constexpr double kEspMost = 1e153;
 __device__ __forceinline__ double esp_coord(double v) {
-  return isfinite(v) ? fmin(fmax(v, -1e100), 1e100) : v;
+  return isfinite(v) ? fmin(fmax(v, -kEspMost), kEspMost) : v;
 }
 
 // Sphere around the finite points of a block of kEspThreads threads with P
@@ -548,16 +550,20 @@ __global__ void __launch_bounds__(kEspThreads, 7)
     if (live[p]) part[(int64_t)y * n + ip[p]] = acc[p];
 }
 
-// V = sum_A Z_A / |C - R_A| - (sum of the rows of part, in row order).
+// V = sum_A Z_A / |C - R_A| - (sum of the rows of part, in row order).  Beyond
+// kEspMost the electronic part is zero; at infinity only with s functions alone
+// (the higher multipoles are infinity times zero there: NaN).
 __global__ void __launch_bounds__(256)
     esp_finish_kernel(const double* __restrict__ part, int rows, const double* __restrict__ atoms, int natom,
-                      const double* __restrict__ xyz, const int32_t* __restrict__ perm, int64_t n,
+                      const double* __restrict__ xyz, const int32_t* __restrict__ perm, int64_t n, bool s_only,
                       double* __restrict__ out) {
   const int64_t ip = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (ip >= n) return;
   const double cx = xyz[ip], cy = xyz[n + ip], cz = xyz[2 * n + ip];
   double elec = 0.0;
   for (int r = 0; r < rows; ++r) elec += part[(int64_t)r * n + ip];
+  const double most = fmax(fmax(fabs(cx), fabs(cy)), fabs(cz));  // (fmax drops a NaN)
+  if (most > kEspMost && (s_only || most < INFINITY) && !isnan(cx) && !isnan(cy) && !isnan(cz)) elec = 0.0;
   double nuc = 0.0;
   for (int a = 0; a < natom; ++a) {
     const double dx = cx - atoms[4 * a], dy = cy - atoms[4 * a + 1], dz = cz - atoms[4 * a + 2];
@@ -923,6 +929,7 @@ static int build_esp(ctc_molecule* mol) {
   if (!pairs.empty()) e->mean_L /= (double)pairs.size();
   e->npairs = (int)pairs.size();
   e->nbatch = (int)batches.size();
+  e->s_only = batches.empty() || batches.back().L == 0;
   e->natom = mol->natom;
   e->nh = hh.size();
   auto up = [&](void** dst, const void* src, size_t bytes) -> int {
@@ -1033,7 +1040,7 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
       else esp_near_kernel<1><<<ngrid, kEspThreads, 0, st>>>(e->d_pairs, e->d_h, e->d_far, e->d_batches, e->nbatch, e->d_boys, xyz, m, near);
       CTC_CUDA_TRY(cudaGetLastError());
     }
-    esp_finish_kernel<<<g, 256, 0, st>>>(part, S + SN, e->d_atoms, e->natom, xyz, perm, m, d_out + p0);
+    esp_finish_kernel<<<g, 256, 0, st>>>(part, S + SN, e->d_atoms, e->natom, xyz, perm, m, e->s_only, d_out + p0);
     CTC_CUDA_TRY(cudaGetLastError());
   }
   return CTC_OK;
