@@ -1,5 +1,6 @@
-// ctc_chunk.h -- how many tiles a chunk of the tile pipeline takes, and when the
-// driver is asked for the free memory first (host arithmetic only).
+// ctc_chunk.h -- host-side rules of the tile pipeline (arithmetic only): how many
+// tiles a chunk takes and when the driver is asked for the free memory first;
+// whether and how finely points are sorted along a Morton curve.
 #pragma once
 
 #include <algorithm>
@@ -23,5 +24,21 @@ inline int64_t chunk_tiles(size_t budget, size_t tile_bytes, int64_t ntiles, int
 // one that fits what the molecule holds already.  (The question takes 0.1 to 6 ms
 // on a shared host, as long as a whole call of 1e5 points.)
 inline bool ask_free_memory(size_t block, size_t held) { return block > std::max(held, kSmallAo); }
+
+// Bits per axis of the Morton keys of points over a box of edge ext (bohr).  Cells
+// of 1/256 of the box are well below a tile's size for most molecules (0.14 bohr
+// for 12 atoms), and 24 bits take three passes of the radix sort instead of four
+// (30 000 points of 12 to 60 atoms: 1 to 8% of the call).  Beyond 512 bohr such a
+// cell is wider than 2 bohr and holds whole tiles' worth of unordered points: on a
+// chain of 500 bohr 24 and 30 bits take the same time (200 000 points on
+// tensor cores: 1.00 and, all at one end, 1.02 of the 30-bit time), on one of 1 500
+// bohr 24 bits cost 5 to 11% more.
+inline int morton_axis_bits(double ext) { return ext <= 512.0 ? 8 : 10; }
+
+// Are explicit points sorted at all?  A basis of up to 256 functions at up to
+// 2 048 points is not: its tiles keep most functions in any order, and the sort's
+// two launches take as long as the rest (200 points of a 160-function molecule: 12
+// of 60 us).
+inline bool sort_points(int64_t n, int mpad, double ext) { return n > 2048 || mpad > 256; }
 
 }  // namespace ctc

@@ -994,10 +994,13 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
     // kernel at 1e5 surface points of 100 atoms: 40 -> 26 ms)
     const int SN = std::min(4 * S, e->nbatch);
     const bool sort = m > kEspThreads;
+    double lo[3], ext = 0;
+    morton_box(mol, lo, &ext);
+    const int bits = morton_axis_bits(ext);
     size_t tmp_bytes = 0;
     if (sort)
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                                   (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, kMortonSortBits, st));
+                                                   (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, 3 * bits, st));
     // One layout gives both the size of the block and the places in it (S and SN
     // are zero when no pair is kept; the finish kernel then reads no row).
     double *part = nullptr, *xyz = nullptr;
@@ -1021,12 +1024,10 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
     lay_out((char*)mol->ws_esp.p);
     const unsigned g = (unsigned)((m + 255) / 256);
     if (sort) {
-      double lo[3], ext = 0;
-      morton_box(mol, lo, &ext);
-      morton_kernel<<<g, 256, 0, st>>>(pts, m, lo[0], lo[1], lo[2], kMortonCells / ext, k_in, v_in);
+      morton_kernel<<<g, 256, 0, st>>>(pts, m, lo[0], lo[1], lo[2], (1 << bits) / ext, bits, k_in, v_in);
       CTC_CUDA_TRY(cudaGetLastError());
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k_in, k_out, v_in, perm, (int)m, 0,
-                                                   kMortonSortBits, st));
+                                                   3 * bits, st));
     }
     esp_gather_kernel<<<g, 256, 0, st>>>(pts, perm, m, xyz);
     CTC_CUDA_TRY(cudaGetLastError());

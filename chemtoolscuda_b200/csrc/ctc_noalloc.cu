@@ -96,15 +96,16 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
   const int TP = fp64_tile_points(plan, n);
   const int64_t ntiles = (n + TP - 1) / TP;
 
-  // Morton order of the points over the molecule's box padded by 12 bohr,
-  // the same ordering ctc_eval_local uses.
+  // Morton order of the points over the molecule's box padded by 12 bohr, at
+  // every size (ctc_eval_local leaves small calls unsorted and packs large ones
+  // sort-tile-recursively).
   double lo[3], ext = 0;
   morton_box(mol, lo, &ext);
+  const int bits = morton_axis_bits(ext);
   size_t sort_tmp = 0;
   CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_tmp, (uint32_t*)nullptr,
                                                (uint32_t*)nullptr, (int32_t*)nullptr,
-                                               (int32_t*)nullptr, (int)n, 0, kMortonSortBits,
-                                               st));
+                                               (int32_t*)nullptr, (int)n, 0, 3 * bits, st));
   Carve cv{(char*)base};
   uint32_t* k_in = cv.take<uint32_t>(n);
   uint32_t* k_out = cv.take<uint32_t>(n);
@@ -156,10 +157,10 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
   }
 
   morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_points, n, lo[0], lo[1], lo[2],
-                                                              kMortonCells / ext, k_in, v_in);
+                                                              (1 << bits) / ext, bits, k_in, v_in);
   CTC_CUDA_TRY(cudaGetLastError());
   CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, sort_tmp, k_in, k_out, v_in, perm, (int)n, 0,
-                                               kMortonSortBits, st));
+                                               3 * bits, st));
   mol->host_launches += 2;
   for (int64_t t0 = 0; t0 < ntiles; t0 += C) {
     tb.C = (int)std::min<int64_t>(C, ntiles - t0);

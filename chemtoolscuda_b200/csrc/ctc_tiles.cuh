@@ -52,30 +52,24 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   return v;
 }
 
-// 24-bit Morton key of each point (the single-sort order of small calls and
-// of the fixed-scratch entry point, ctc_noalloc.cu); a point with a
-// non-finite coordinate gets
-// kNonFiniteKey, the last one, so the sort puts such points behind the others
-// (but for points in the box's last cell).  Cells of 1/256 of the box (0.14 bohr
-// for 12 atoms) are well below a tile's size for the calls that use this order,
-// and 24 bits take three passes of the radix sort instead of four.
-constexpr uint32_t kNonFiniteKey = (1u << 24) - 1u;
-constexpr int kMortonCells = 256;
-constexpr int kMortonSortBits = 24;
-
+// Morton key of each point, `bits` bits per axis (the single-sort order of small
+// calls and of the fixed-scratch entry point, ctc_noalloc.cu; morton_axis_bits).
+// A point with a non-finite coordinate gets the last key, so the sort puts such
+// points behind the others (but for points in the box's last cell).
 __global__ void morton_kernel(const double* __restrict__ pts, int64_t n, double lox, double loy,
-                              double loz, double inv_cell, uint32_t* keys, int32_t* vals) {
+                              double loz, double inv_cell, int bits, uint32_t* keys, int32_t* vals) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  const double last = (double)((1 << bits) - 1);
   auto q = [&](double v, double lo) {
     double c = (v - lo) * inv_cell;
-    c = c < 0.0 ? 0.0 : (c > kMortonCells - 1.0 ? kMortonCells - 1.0 : c);
+    c = c < 0.0 ? 0.0 : (c > last ? last : c);
     return (uint32_t)c;
   };
   const double x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
-  keys[i] = isfinite(x) && isfinite(y) && isfinite(z)
+  keys[i] = finite_point(pts + 3 * i)
                 ? spread10(q(x, lox)) | (spread10(q(y, loy)) << 1) | (spread10(q(z, loz)) << 2)
-                : kNonFiniteKey;
+                : (1u << 3 * bits) - 1u;
   vals[i] = (int32_t)i;
 }
 
@@ -581,22 +575,22 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
   }
   int rc;
   // explicit points: sort-tile-recursive order over the points' own box for
-  // calls of kStrMinPoints points or more; below that, one sort of 24-bit
-  // Morton keys over the molecule's box padded by 12 bohr (three sorts cost
-  // ~0.4 ms, as much as a whole 1e5-point density call of a small molecule,
-  // while the tiles' shape matters little there)
+  // calls of kStrMinPoints points or more; below that, one sort of Morton keys
+  // over the molecule's box padded by 12 bohr (three sorts cost ~0.4 ms, as much
+  // as a whole 1e5-point density call of a small molecule, while the tiles' shape
+  // matters little there), or none (sort_points)
   constexpr int64_t kStrMinPoints = (int64_t)1 << 18;
   int32_t* perm = nullptr;
-  // A basis of up to 256 functions at up to 2 048 points is not sorted: its tiles
-  // keep most functions in any order, and the sort's two launches take as long as
-  // the rest (200 points of a 160-function molecule: 12 of 60 us).
-  if (!src.cubic && (n > 2048 || mol->Mpad > 256)) {
+  double lo[3], ext = 0;
+  if (!src.cubic) morton_box(mol, lo, &ext);
+  if (!src.cubic && sort_points(n, mol->Mpad, ext)) {
     const bool str = n >= kStrMinPoints;
+    const int bits = morton_axis_bits(ext);
     size_t tmp_bytes = 0, tmp32 = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint64_t*)nullptr, (uint64_t*)nullptr,
                                     (int32_t*)nullptr, (int32_t*)nullptr, (int)n, 0, 64, st);
     cub::DeviceRadixSort::SortPairs(nullptr, tmp32, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                    (int32_t*)nullptr, (int32_t*)nullptr, (int)n, 0, kMortonSortBits, st);
+                                    (int32_t*)nullptr, (int32_t*)nullptr, (int)n, 0, 3 * bits, st);
     tmp_bytes = std::max(tmp_bytes, tmp32);
     const size_t need = 2 * sizeof(uint64_t) * (size_t)n + 2 * sizeof(int32_t) * (size_t)n + tmp_bytes + 4096;
     if ((rc = mol->ws_part.ensure(need, st)) != CTC_OK) return rc;
@@ -623,15 +617,13 @@ inline int run_tiles(ctc_molecule* mol, const PointSrc& src, int64_t n, int TP, 
       }
       mol->host_launches += 7;
     } else {
-      double lo[3], ext = 0;
-      morton_box(mol, lo, &ext);
       uint32_t* k32_in = (uint32_t*)k_in;
       uint32_t* k32_out = (uint32_t*)k_out;
-      morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src.pts, n, lo[0], lo[1], lo[2], kMortonCells / ext,
-                                                                  k32_in, v_in);
+      morton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src.pts, n, lo[0], lo[1], lo[2], (1 << bits) / ext,
+                                                                  bits, k32_in, v_in);
       CTC_CUDA_TRY(cudaGetLastError());
       CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k32_in, k32_out, v_in, perm, (int)n, 0,
-                                                   kMortonSortBits, st));
+                                                   3 * bits, st));
       mol->host_launches += 2;
     }
   }
