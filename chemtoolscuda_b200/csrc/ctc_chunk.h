@@ -36,9 +36,11 @@ inline bool ask_free_memory(size_t block, size_t held) { return block > std::max
 inline int morton_axis_bits(double ext) { return ext <= 512.0 ? 8 : 10; }
 
 // Are explicit points sorted at all?  A basis of up to 256 functions at up to
-// 2 048 points is not: its tiles keep most functions in any order, and the sort's
-// two launches take as long as the rest (200 points of a 160-function molecule: 12
-// of 60 us).
-inline bool sort_points(int64_t n, int mpad, double ext) { return n > 2048 || mpad > 256; }
+// 2 048 points is not, unless its atoms lie far apart (box beyond 64 bohr, 24 of
+// them padding): its tiles keep most functions in any order, and the sort's two
+// launches take as long as the rest (a call of 100 to 2 048 points unsorted, of its
+// time sorted: 6 to 20 atoms 0.68 to 0.96, chain of 40 bohr 0.81 to 1.04, of 70 bohr
+// 0.78 to 1.21, of 170 bohr 0.94 to 1.42).
+inline bool sort_points(int64_t n, int mpad, double ext) { return n > 2048 || mpad > 256 || !(ext <= 64.0); }
 
 }  // namespace ctc

@@ -58,3 +58,11 @@ def test_cells(rules):
         assert bits in (8, 10)  # 24 or 30 bits in all: spread10 and 32-bit keys hold both
         assert ext / 2 ** bits <= max(2.0, ext / 1024)
     assert rules.axis_bits(float("nan")) == 10
+
+
+def test_small_calls_of_spread_out_molecules_are_sorted(rules):
+    """Unsorted only where a tile keeps most functions in any order: few points, few
+    functions, and a molecule of at most 40 bohr (64 with its padding)."""
+    assert not rules.sorted(2048, 256, 64.0) and not rules.sorted(1, 128, 24.0)
+    assert rules.sorted(2049, 128, 24.0) and rules.sorted(1, 384, 24.0)
+    assert rules.sorted(1, 128, 64.1) and rules.sorted(2048, 256, 1000.0) and rules.sorted(1, 128, float("nan"))
