@@ -61,3 +61,27 @@ def test_number_of_items_does_not_change_results(torch_cuda, keys):
         for k in keys:
             w = whole[k].reshape(shape[0], -1)[x0:x0 + nx].ravel()
             assert np.array_equal(part[k], w), k
+
+
+@pytest.mark.parametrize("keys,per_tile", [(("rho",), 128), (KEYS, 32)])
+@pytest.mark.parametrize("near,far", [(1, 140), (12, 90), (40, 40)])
+def test_tiles_of_very_different_sizes(torch_cuda, keys, per_tile, near, far):
+    """Tiles near the molecule (several slices, cut into up to eight items) among
+    tiles that keep few functions or none, whose further items are empty."""
+    mol = S.make_molecule("c2", seed=6, natom=30, box=11.0, nocc=60)
+    rng = np.random.default_rng(near)
+    pts = np.concatenate([S.random_points(rng, mol, near * per_tile, pad=0.5),
+                          mol.coords.mean(0) + np.array([22.0, 0.0, 0.0]) + rng.uniform(-9, 9, (far * per_tile, 3))])
+    m = ctc_abi.Mol(mol.flat(), mol.coords, mol.charges, mol.D)
+    few = np.r_[0:min(100, near * per_tile), len(pts) - 50:len(pts)]
+    ref = O.eval_local(mol.flat(), mol.D, pts[few], alpha=0.5, keys=KEYS)
+    sc = term_scales(mol.flat(), mol.D, pts[few], alpha=0.5)
+    first = m.eval_local(pts, keys, ctc_abi.PREC_TC)
+    for k in keys:
+        assert np.isfinite(first[k]).all()
+        assert_close(k, first[k][few], ref[k], sc[k], 1e-8, atol=1e-15)
+    for _ in range(50):
+        again = m.eval_local(pts, keys, ctc_abi.PREC_TC)
+        for k in keys:
+            assert np.array_equal(again[k], first[k])
+    assert m.sync_status() == 0
