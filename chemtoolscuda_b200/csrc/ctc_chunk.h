@@ -13,11 +13,14 @@ namespace ctc {
 // less), and the block that is taken without asking how much is free.
 constexpr size_t kMostAo = (size_t)12 << 30, kSmallAo = (size_t)64 << 20;
 
-// Tiles of a chunk: what the budget holds and at least one per SM; a call of
-// several chunks takes whole rounds of one tile per SM.
+// Tiles of a chunk: what the budget holds and at least one per SM.  A call of
+// several chunks takes whole rounds of one tile per SM where that drops at most a
+// twentieth of the chunk (1 787 -> 1 776 tiles, FP64 contraction of the 90 945-point
+// cube of 200 atoms: call 33.5 -> 33.2 ms; the tensor-core form, which deals out
+// items, 78.0 either way; 714 -> 592 would make eleven chunks of nine).
 inline int64_t chunk_tiles(size_t budget, size_t tile_bytes, int64_t ntiles, int sms) {
   const int64_t C = std::min<int64_t>(std::max<int64_t>(sms, (int64_t)(budget / tile_bytes)), ntiles);
-  return C < ntiles ? C - C % sms : C;
+  return C < ntiles && C % sms <= C / 20 ? C - C % sms : C;
 }
 
 // The free memory matters only to a block that has still to be allocated: not to
