@@ -208,16 +208,17 @@ def load_lib():
 
 def esp_roofline(lib, h, points, ms, fp64_peak):
     """FP64-pipe roofline of the ESP kernels (far pairs, near pairs, then the
-    fixed-order sum): algorithmic FP64 operations per point (ctc_molecule_esp_info)
-    x points / the call's device time, against the measured FP64 peak."""
+    fixed-order sum): FP64 operations per point with every pair in its far-field
+    form (ctc_molecule_esp_info; near pairs cost more) x points / the call's device
+    time, against the measured FP64 peak."""
     info = (C.c_double * 4)()
     check(lib, lib.ctc_molecule_esp_info(h, info), "esp_info")
     achieved = info[1] * points / (ms * 1e-3) / 1e12
-    return {"kernel": "esp_far_kernel (point multipoles) + esp_near_kernel (Boys function) + esp_finish_kernel; the work formula counts the R recursion for every pair", "bound": "fp64",
+    return {"kernel": "esp_far_kernel (point multipoles) + esp_near_kernel (Boys function) + esp_finish_kernel", "bound": "fp64",
             "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s (fp64)", "frac": achieved / fp64_peak,
             "peak_source": "measured (cuBLAS DGEMM 8192^3, burst)",
             "flops_per_point": info[1], "primitive_pairs": info[0], "mean_L": info[3],
-            "work_formula": "per kept primitive pair: 2 n_tuv(L) + 2 n_R(L) + 10 (L+1)"}
+            "work_formula": "per kept primitive pair, far form: 18 (L = 0), 26 (L = 1), 20 + 2 n_tuv(L); near pairs cost more"}
 
 
 def check(lib, rc, what):

@@ -103,6 +103,10 @@ __host__ __device__ constexpr int nnear(int L) {
 // 16-byte loads
 __host__ __device__ constexpr int nfar(int L) { return ntuv(L) / 2 * 2; }
 
+// FP64 operations of esp_far_pair per pair and point, a multiply-add counted as two:
+// P - C and its square 8, the root 8, the last multiply-add 2, and the polynomial.
+__host__ __device__ constexpr int far_flops(int L) { return L == 0 ? 18 : (L == 1 ? 26 : 20 + 2 * ntuv(L)); }
+
 double boys_series(int m, double T) {
   double term = 1.0 / (2 * m + 1), sum = term;
   for (int i = 1; i < 1000; ++i) {
@@ -133,8 +137,8 @@ struct EspTables {
   int npairs = 0, nbatch = 0, natom = 0;
   bool s_only = false;        // every kept pair is of class 0
   size_t nh = 0;
-  // algorithmic FP64 work per point: sum over the kept pairs of
-  // 2 n_tuv(L) (contraction) + 2 n_R(L) (R recursion) + 10 (L + 1) (Boys)
+  // FP64 work per point with every kept pair in its far form (far_flops): what the
+  // call cannot do without, as a near pair costs more
   double flops_per_point = 0.0;
   double mean_L = 0.0;
 };
@@ -920,10 +924,8 @@ static int build_esp(ctc_molecule* mol) {
   EspTables* e = new EspTables();
   mol->esp = e;
   for (const EspBatch& bt : batches) {
-    int nR = 0;
-    for (int j = 0; j <= bt.L; ++j) nR += ntuv(j);
     const int np = bt.b1 - bt.b0;
-    e->flops_per_point += (double)np * (2.0 * ntuv(bt.L) + 2.0 * nR + 10.0 * (bt.L + 1));
+    e->flops_per_point += (double)np * far_flops(bt.L);
     e->mean_L += (double)np * bt.L;
   }
   if (!pairs.empty()) e->mean_L /= (double)pairs.size();

@@ -233,10 +233,11 @@ int ctc_eval_esp_host(ctc_molecule* mol, const double* h_points, int64_t npoints
 
 /* Work of the ESP evaluation (no counterpart in the reference; builds the
  * molecule's pair tables if needed): info[0] primitive pairs kept after the
- * point-independent screening, [1] algorithmic FP64 operations per point,
- * sum over those pairs of 2 n_tuv(L) + 2 n_R(L) + 10 (L + 1) with
- * n_tuv(L) = (L+1)(L+2)(L+3)/6 and n_R(L) = sum_{j<=L} n_tuv(j), [2] Hermite
- * coefficients stored, [3] mean L = l_a + l_b of the kept pairs. */
+ * point-independent screening, [1] FP64 operations per point with every pair in
+ * its far-field form (a multiply-add counted as two; near pairs cost more): 18
+ * for L = 0, 26 for L = 1, 20 + 2 n_tuv(L) beyond, with
+ * n_tuv(L) = (L+1)(L+2)(L+3)/6, [2] Hermite coefficients formed, [3] mean
+ * L = l_a + l_b of the kept pairs. */
 int ctc_molecule_esp_info(ctc_molecule* mol, double* info /* [4] */);
 
 /* ---- adjoint (no counterpart in the reference) --------------------------------------------- */
