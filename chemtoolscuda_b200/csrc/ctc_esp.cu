@@ -348,7 +348,10 @@ __device__ int esp_select(const EspPair* __restrict__ pairs, int np, const doubl
 
 // 1 / sqrt(x): the hardware's approximation (relative error below 2^-19 over
 // the normal range) and one step of Householder's third-order iteration, whose
-// remainder is (5/16) e^3 < 2^-55 (measured: 1.4e-16; rsqrt(): 1.1e-16).
+// remainder is (5/16) e^3 < 2^-55 (measured: 1.4e-16; rsqrt(): 1.1e-16).  With
+// rsqrt() 1e5 surface points of 100 atoms take 149.3 ms instead of 136.7, 1 500
+// points of 12 atoms 270 us instead of 260, and the potential's error against 64
+// bits is the same (1.3e-15 of its scale).
 __device__ __forceinline__ double esp_rsqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
