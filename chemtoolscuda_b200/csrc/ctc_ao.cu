@@ -281,7 +281,9 @@ int launch_ao_tiles(const ctc_molecule* mol, const TileBatch& tb, int deriv, cud
   // few tiles: their segments on more CTAs, up to twelve for every SM, of which
   // three or more run at a time, so that the last round is a small part (values of
   // 62 segments at 200 points, seven tiles: 18 us on one CTA each, 5.5 on eight)
-  const dim3 grid((unsigned)tb.C, (unsigned)std::max(1, std::min(8, (12 * 148 + tb.C - 1) / tb.C)));
+  int nsm = 0;
+  if (int rc = device_sm_count(&nsm); rc != CTC_OK) return rc;
+  const dim3 grid((unsigned)tb.C, (unsigned)std::max(1, std::min(8, (12 * nsm + tb.C - 1) / tb.C)));
   switch (deriv) {
     case 0: ao_tile_kernel<0, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
     case 1: ao_tile_kernel<1, 0><<<grid, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, nullptr, nullptr, nullptr, nullptr); break;
@@ -306,7 +308,8 @@ int launch_ao_tiles_weighted(const ctc_molecule* mol, const TileBatch& tb, const
 int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int deriv, int nqa,
                            int8_t* planes, int32_t* eexp, const int32_t* order, cudaStream_t st) {
   if (tb.C <= 0) return CTC_OK;
-  if (!(nqa == 4 && tb.TP == 32 && deriv >= 1) && !(nqa == 1 && tb.TP == 128))
+  // (second derivatives come with four rows per point: plan_local)
+  if (!(nqa == 4 && tb.TP == 32 && deriv >= 1) && !(nqa == 1 && tb.TP == 128 && deriv <= 1))
     return fail(CTC_ERR_INVALID, "sliced AO tiles: unsupported row layout");
   if (planes == nullptr || eexp == nullptr)
     return fail(CTC_ERR_INVALID, "sliced AO tiles: null workspace");
@@ -316,11 +319,8 @@ int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int der
     if (deriv == 1) ao_tile_kernel<1, 4><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
     else ao_tile_kernel<2, 4><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
   } else {
-    switch (deriv) {
-      case 0: ao_tile_kernel<0, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr); break;
-      case 1: ao_tile_kernel<1, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr); break;
-      default: ao_tile_kernel<2, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
-    }
+    if (deriv == 0) ao_tile_kernel<0, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
+    else ao_tile_kernel<1, 1><<<tb.C, kAoThreads, 0, st>>>(sg, mol->nseg, al, co, tb, eexp, order, nullptr, nullptr);
   }
   CTC_CUDA_TRY(cudaGetLastError());
   slice_rows_kernel<<<tb.C, kSliceThreads, 0, st>>>(tb, nqa, eexp, planes, order);

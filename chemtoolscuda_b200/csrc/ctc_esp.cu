@@ -51,9 +51,7 @@
 
 #include "ctc_tiles.cuh"
 
-#define CTC_TERMS_HOST
 #include "ctc_terms.inc"
-#undef CTC_TERMS_HOST
 
 namespace ctc {
 

@@ -66,26 +66,7 @@ struct PointSrc {
   double ax[9];        // cubic axes, row i = axis i
   int32_t ny, nz;      // cubic shape (x extent implied)
   int32_t cubic;
-  int64_t offset;      // global index of the first point of this launch
 };
-
-__host__ __device__ inline void point_of(const PointSrc& s, int64_t i, double& x, double& y,
-                                         double& z) {
-  int64_t g = s.offset + i;
-  if (s.cubic) {
-    int64_t k = g % s.nz;
-    int64_t j = (g / s.nz) % s.ny;
-    int64_t ii = g / ((int64_t)s.nz * s.ny);
-    double fi = (double)ii, fj = (double)j, fk = (double)k;
-    x = s.o[0] + fi * s.ax[0] + fj * s.ax[3] + fk * s.ax[6];
-    y = s.o[1] + fi * s.ax[1] + fj * s.ax[4] + fk * s.ax[7];
-    z = s.o[2] + fi * s.ax[2] + fj * s.ax[5] + fk * s.ax[8];
-  } else {
-    x = s.pts[3 * g];
-    y = s.pts[3 * g + 1];
-    z = s.pts[3 * g + 2];
-  }
-}
 
 // Device scratch owned by a molecule; grows on demand, released stream-ordered.
 struct Scratch {

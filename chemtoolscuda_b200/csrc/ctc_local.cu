@@ -45,7 +45,9 @@ LocalPlan plan_local(const ctc_outputs* o) {
 // two 128-point tiles for every SM (density at 200 points of a 160-function
 // molecule: 58 us as two tiles of 128, 13 us as seven of 32).
 int fp64_tile_points(const LocalPlan& plan, int64_t n) {
-  return plan.nqa == 4 || n < (int64_t)128 * 148 * 2 ? 32 : 128;
+  int nsm = 0;
+  if (device_sm_count(&nsm) != CTC_OK) return 32;  // (the launches report it)
+  return plan.nqa == 4 || n < (int64_t)128 * nsm * 2 ? 32 : 128;
 }
 
 int fp64_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& tb,

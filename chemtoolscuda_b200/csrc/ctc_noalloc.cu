@@ -92,6 +92,8 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
   // a failure an earlier stream-ordered call recorded on the device
   if ((rc = poll_status(mol, st)) != CTC_OK) return rc;
 
+  int nsm = 0;
+  if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   const LocalPlan plan = plan_local(out);
   const int TP = fp64_tile_points(plan, n);
   const int64_t ntiles = (n + TP - 1) / TP;
@@ -170,7 +172,7 @@ int eval_local_noalloc(ctc_molecule* mol, const double* d_points, int64_t n, con
     screen_kernel<<<tb.C, kTileThreads, 0, st>>>(mol->d_segs, mol->nseg, tb, TP * plan.nqa, mol->d_stats,
                                                  mol->d_status);
     CTC_CUDA_TRY(cudaGetLastError());
-    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb, 148, 0.0);
+    tile_order_kernel<<<1, kOrderThreads, 0, st>>>(tb, nsm, 0.0);
     CTC_CUDA_TRY(cudaGetLastError());
     if ((rc = launch_ao_tiles(mol, tb, plan.deriv, st)) != CTC_OK) return rc;
     if ((rc = fp64_local_tiles(mol, plan, tb, prm, out, st)) != CTC_OK) return rc;

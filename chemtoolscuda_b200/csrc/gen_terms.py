@@ -82,23 +82,14 @@ def main():
         row.append(len(terms))
         offs.append(row + [row[-1]] * (16 - len(row)))
     print("// Generated by gen_terms.py -- do not edit.")
-    print("// Define CTC_TERMS_HOST before including to get host arrays h_terms/h_comp_off")
-    print("// instead of the __constant__ device arrays c_terms/c_comp_off.")
+    print("// (Host arrays: the kernels' angular polynomials are in ctc_ao_poly.inc.)")
     print(f"#define CTC_NTERMS {len(terms)}")
-    print("#ifdef CTC_TERMS_HOST")
     print("static const ctc::Term h_terms[CTC_NTERMS] = {")
-    print("#else")
-    print("__constant__ ctc::Term c_terms[CTC_NTERMS] = {")
-    print("#endif")
     for c, a, b, z in terms:
         print(f"  {{{c!r}, {a}, {b}, {z}, 0}},")
     print("};")
     print("// [type][j] .. [type][j+1] are the terms of component j")
-    print("#ifdef CTC_TERMS_HOST")
     print("static const int16_t h_comp_off[8][16] = {")
-    print("#else")
-    print("__constant__ int16_t c_comp_off[8][16] = {")
-    print("#endif")
     for row in offs:
         print("  {" + ", ".join(str(x) for x in row) + "},")
     print("};")
