@@ -169,6 +169,7 @@ int Scratch::ensure(size_t need, cudaStream_t st) {
   cudaError_t e = cudaMallocAsync(&p, alloc, st);
   if (e != cudaSuccess) {
     p = nullptr;
+    cudaGetLastError();  // else the next launch's check would report this error again
     return fail(CTC_ERR_NOMEM, std::string("scratch allocation of ") + std::to_string(alloc) +
                                    " bytes failed: " + cudaGetErrorString(e));
   }
