@@ -293,12 +293,11 @@ int ctc_eval_esp_host(ctc_molecule* mol, const double* h_points, int64_t n, doub
   if (n < 0) return fail(CTC_ERR_INVALID, "ctc_eval_esp_host: negative point count");
   if (n == 0) return CTC_OK;
   // the device copies of points and results stay with the molecule (up to 32
-  // MiB; larger calls give theirs back)
+  // MiB and within its scratch limit; others are given back)
   const size_t bytes = sizeof(double) * 4 * (size_t)n;
-  const bool keep = bytes <= (size_t)32 << 20;
+  const bool keep = bytes <= (size_t)32 << 20 && mol->ws_io.ensure(bytes, 0) == CTC_OK;
   double* d = nullptr;
   if (keep) {
-    if (int rc = mol->ws_io.ensure(bytes, 0); rc != CTC_OK) return rc;
     d = (double*)mol->ws_io.p;
   } else if (cudaMalloc((void**)&d, bytes) != cudaSuccess) {
     cudaGetLastError();

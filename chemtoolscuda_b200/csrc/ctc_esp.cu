@@ -980,40 +980,30 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
   const EspTables* e = mol->esp;
   int nsm = 148;
   if (int rc = device_sm_count(&nsm); rc != CTC_OK) return rc;
+  double lo[3], ext = 0;
+  morton_box(mol, lo, &ext);
+  const int bits = morton_axis_bits(ext);
   // points per pass: bounds the partial-sum rows (rows x points x 8 B)
-  constexpr int64_t kChunk = (int64_t)1 << 22;
-  for (int64_t p0 = 0; p0 < n; p0 += kChunk) {
-    const int64_t m = std::min(kChunk, n - p0);
+  int64_t pass = (int64_t)1 << 22;
+  int most_slices = 16383;  // (four times as many fit the grid's y)
+  int near_factor = 4;
+  for (int64_t p0 = 0, m = 0; p0 < n; p0 += m) {
     const double* pts = d_points + 3 * p0;
-    // two points per thread share a pair's coefficients; one when the points
-    // would fill less than a block per SM (the pairs are then cut into more
-    // slices)
-    const int P = m >= (int64_t)2 * kEspThreads * nsm ? 2 : 1;
-    const int64_t gx = (m + P * kEspThreads - 1) / (P * kEspThreads);
-    // slices of the batches: about 32 blocks per SM, at least a batch each
-    const int64_t want = (32 * (int64_t)nsm + gx - 1) / gx;
-    const int S = e->nbatch == 0 ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)e->nbatch, 16383}));
-    // near pairs cluster in few batches: four times as many slices for them (near
-    // kernel at 1e5 surface points of 100 atoms: 40 -> 26 ms)
-    const int SN = std::min(4 * S, e->nbatch);
-    const bool sort = m > kEspThreads;
-    double lo[3], ext = 0;
-    morton_box(mol, lo, &ext);
-    const int bits = morton_axis_bits(ext);
+    int P = 1, S = 0, SN = 0;
+    int64_t gx = 0;
+    bool sort = false;
     size_t tmp_bytes = 0;
-    if (sort)
-      CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                                   (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, 3 * bits, st));
-    // One layout gives both the size of the block and the places in it (S and SN
-    // are zero when no pair is kept; the finish kernel then reads no row).
     double *part = nullptr, *xyz = nullptr;
     uint32_t *k_in = nullptr, *k_out = nullptr;
     int32_t *v_in = nullptr, *perm = nullptr;
     void* tmp = nullptr;
+    // One layout gives both the size of the block and the places in it (S and SN
+    // are zero when no pair is kept; the finish kernel then reads no row).
     auto lay_out = [&](char* base) {
       Carve cv{base};
       part = cv.take<double>((size_t)(S + SN) * m);
       xyz = cv.take<double>(3 * (size_t)m);
+      perm = nullptr;  // (a larger pass that did not fit may have been sorted)
       if (sort) {
         k_in = cv.take<uint32_t>(m);
         k_out = cv.take<uint32_t>(m);
@@ -1023,7 +1013,33 @@ int eval_esp(ctc_molecule* mol, const double* d_points, int64_t n, double* d_out
       }
       return cv.off;
     };
-    if (int rc = mol->ws_esp.ensure(lay_out(nullptr), st); rc != CTC_OK) return rc;
+    for (;;) {
+      m = std::min(pass, n - p0);
+      // two points per thread share a pair's coefficients; one when the points
+      // would fill less than a block per SM (the pairs are then cut into more
+      // slices)
+      P = m >= (int64_t)2 * kEspThreads * nsm ? 2 : 1;
+      gx = (m + P * kEspThreads - 1) / (P * kEspThreads);
+      // slices of the batches: about 32 blocks per SM, at least a batch each
+      const int64_t want = (32 * (int64_t)nsm + gx - 1) / gx;
+      S = e->nbatch == 0 ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)e->nbatch, (int64_t)most_slices}));
+      // near pairs cluster in few batches: four times as many slices for them (near
+      // kernel at 1e5 surface points of 100 atoms: 40 -> 26 ms)
+      SN = std::min(near_factor * S, e->nbatch);
+      sort = m > kEspThreads;
+      if (sort)
+        CTC_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                                     (int32_t*)nullptr, (int32_t*)nullptr, (int)m, 0, 3 * bits, st));
+      const int rc = mol->ws_esp.ensure(lay_out(nullptr), st);
+      if (rc == CTC_OK) break;
+      // no room: fewer slices, then fewer points per pass (the sums' order follows
+      // the slices, so results then differ in the last bits)
+      if (rc != CTC_ERR_NOMEM) return rc;
+      if (S > 1) most_slices = S / 2;
+      else if (near_factor > 1) near_factor = 1;
+      else if (m > kEspThreads) pass = std::max<int64_t>(kEspThreads, m / 2);
+      else return rc;
+    }
     lay_out((char*)mol->ws_esp.p);
     const unsigned g = (unsigned)((m + 255) / 256);
     if (sort) {
