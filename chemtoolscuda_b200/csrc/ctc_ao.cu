@@ -332,8 +332,13 @@ int launch_ao_tiles_sliced(const ctc_molecule* mol, const TileBatch& tb, int der
 template <int DERIV>
 static int launch_ao_pub(const ctc_molecule* mol, const double* pts, int64_t n, double* out, cudaStream_t st) {
   if (int rc = ensure_smem_attr((const void*)ao_public_kernel<DERIV>, (int)ao_pub_smem(DERIV)); rc != CTC_OK) return rc;
-  const int k = DERIV == 2 ? 1 : 0;
-  const int64_t items = (n + 31) / 32 * mol->n_aochunk[k];
+  int nsm = 0;
+  if (int rc = device_sm_count(&nsm); rc != CTC_OK) return rc;
+  // few points: the narrower chunks, on more CTAs (values at one or two points of 60
+  // to 200 atoms: 12.2 us, 10.4 with them)
+  const int64_t groups = (n + 31) / 32;
+  const int k = DERIV == 2 || groups * mol->n_aochunk[0] < nsm ? 1 : 0;
+  const int64_t items = groups * mol->n_aochunk[k];
   ao_public_kernel<DERIV><<<(unsigned)std::min<int64_t>(items, INT32_MAX), kAoPubThreads, ao_pub_smem(DERIV), st>>>(
       mol->d_segs, mol->d_order, mol->d_aochunk[k], mol->n_aochunk[k], mol->nseg, mol->d_alpha, mol->d_coef, pts, n,
       mol->M, out);
