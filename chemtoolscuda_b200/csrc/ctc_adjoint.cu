@@ -194,10 +194,18 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
   const int nq = v_grad ? (dLdR ? 11 : 2) : (dLdR ? 4 : 1);
   const int deriv = dLdR ? 1 : 0;               // without v_grad
   const int wq = v_grad ? (dLdR ? 10 : 1) : 0;  // quantity of w, 0: none
-  const int TP = dLdR && v_grad ? fp64_points(kFForce2) : fp64_points(kFForce1);
+  int nsm = 148;
+  int rc;
+  if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
+  // Two rows per point: tiles of 64 points, and of 32 while every tile then has an
+  // SM of its own.  The longest tile's time is the call's, and a tile of fewer
+  // points keeps no more functions (dL/dR at 64 points of a 300-bohr chain of 100
+  // atoms: 1 906 us as one tile, 947 as two; 3 000 points of 60 atoms 1 073 and 846;
+  // from 32 points per SM on the second round of tiles takes it back).
+  const int TP = !(dLdR && v_grad) ? fp64_points(kFForce1)
+                                   : (n <= (int64_t)32 * nsm ? fp64_points(kFForce2S) : fp64_points(kFForce2));
   const int Mpad = mol->Mpad;
   double* Cacc = nullptr;
-  int rc;
   if (dLdD) {
     // accumulator of S = A^T W + W^T A (upper triangle used)
     const size_t cbytes = sizeof(double) * (size_t)Mpad * Mpad;
@@ -214,8 +222,6 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
   const std::function<int(const TileBatch&)> weighted = [&](const TileBatch& tb) {
     return launch_ao_tiles_weighted(mol, tb, v_rho, v_grad, st);
   };
-  int nsm = 148;
-  if ((rc = device_sm_count(&nsm)) != CTC_OK) return rc;
   rc = run_tiles(mol, src, n, TP, nq, deriv, st, [&](const TileBatch& tb) -> int {
     if (dLdD) {
       int r2;
@@ -228,7 +234,8 @@ int eval_adjoint(ctc_molecule* mol, const double* d_points, int64_t n, const dou
       mol->host_launches += 2;
     }
     if (dLdR) {
-      const int r3 = v_grad ? launch_fp64<kFForce2>(mol, tb, fa, st) : launch_fp64<kFForce1>(mol, tb, fa, st);
+      const int r3 = !v_grad ? launch_fp64<kFForce1>(mol, tb, fa, st)
+                     : tb.TP == 32 ? launch_fp64<kFForce2S>(mol, tb, fa, st) : launch_fp64<kFForce2>(mol, tb, fa, st);
       if (r3 != CTC_OK) return r3;
       mol->host_launches += 1;
     }

@@ -30,7 +30,7 @@
 //     points: 70.8 -> 36.2 ms;  60 atoms (820), 20 011 points: 2.97 -> 1.39 ms
 //   density, 12 atoms (160), 100 000 points: 276 -> 127 us; 200 points: 58 -> 13 us
 //   rho and gradient (full sums), 60 atoms, 268 800 points: 10.1 -> 7.1 ms
-//   dL/dR, same points: 60.8 -> 15.8 ms
+//   dL/dR, same points: 60.8 -> 15.8 ms; 64 points: 1 830 -> 834 us (tiles of 32)
 //
 // Every barrier wait is bounded (ctc_molecule_set_wait_limit): after the limit a
 // role sets the CTA's abort flag and stops, the others' waits run out in turn, and
@@ -69,9 +69,10 @@ enum Fp64Mode {
   kFSmall1 = 2,   // 32 points x phi, local descriptors (few tiles: more CTAs busy)
   kFForce2 = 3,   // 64 points x {phi, w}, dL/dR with dL/d(grad rho)
   kFForce1 = 4,   // 128 points x phi, dL/dR without it
+  kFForce2S = 5,  // 32 points x {phi, w}: kFForce2 for few points
 };
 constexpr int fp64_points(int mode) {
-  return mode == kFLocal4 || mode == kFSmall1 ? 32 : (mode == kFForce2 ? 64 : 128);
+  return mode == kFLocal4 || mode == kFSmall1 || mode == kFForce2S ? 32 : (mode == kFForce2 ? 64 : 128);
 }
 
 struct Fp64Args {
@@ -228,7 +229,9 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
   constexpr int PTS = fp64_points(MODE);
   constexpr bool NARROW_ONLY = MODE == kFSmall1;
   constexpr bool HAS_NARROW = MODE == kFLocal4 || MODE == kFSmall1;
-  constexpr bool FORCE = MODE == kFForce1 || MODE == kFForce2;
+  constexpr bool FORCE2 = MODE == kFForce2 || MODE == kFForce2S;
+  constexpr bool FORCE = MODE == kFForce1 || FORCE2;
+  constexpr int ROWS = FORCE2 ? 2 * PTS : kFRows;  // rows of a wide stage in use
   extern __shared__ __align__(16) double fsmem[];
   double* sA = fsmem;
   double* sB = fsmem + kFStages * kFAStage;
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
       {
         const double* A = tb.ao + (int64_t)cur.t * nq_ao * ldq + (int64_t)cur.kb * kFK * PTS;
         const bool wide = !NARROW_ONLY && cur.kb < cur.wide;
-        constexpr int NRUN = MODE == kFLocal4 ? 4 : (MODE == kFForce2 ? 2 : 1);  // quantities of a wide stage
+        constexpr int NRUN = MODE == kFLocal4 ? 4 : (FORCE2 ? 2 : 1);  // quantities of a wide stage
         const int runs = wide ? NRUN : 1;
         if (lane == 0) {
           s_issued[s][khalf] = it;
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
         __syncwarp();
         for (int x = lane; x < 16 * runs; x += 32) {
           const int kk = 16 * khalf + x / runs, r = x % runs;
-          const int q = MODE == kFForce2 ? 10 * r : r;
+          const int q = FORCE2 ? 10 * r : r;
           bulk_copy(a + kk * kFALd + r * PTS, A + q * ldq + (int64_t)kk * PTS, PTS * 8, &tma_bar[s]);
         }
       }
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
       for (int nt = 0; nt < nn && !stop; ++nt, ++gs) {
         const FSlice fs = fslice<MODE>(nt, nk, tri, nq_ao);
         const int ncol = min(kFN, nk * kFK - nt * kFN);  // 32 or 64
-        const bool on_w = wn * 32 < ncol, on_n = w * 8 < ncol;
+        const bool on_w = wn * 32 < ncol && wm * 32 < ROWS, on_n = w * 8 < ncol;
         double c[4][4][2];  // wide accumulators
         double d[4][2];     // narrow: rows 0..31, columns w * 8 ..
 #pragma unroll
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
           const int64_t oi = tb.out[p];
           const bool ok = oi >= 0;
           vr[h] = ok ? args.v_rho[oi] : 0.0;
-          for (int k = 0; k < 3; ++k) vg[h][k] = ok && MODE == kFForce2 ? args.v_grad[3 * oi + k] : 0.0;
+          for (int k = 0; k < 3; ++k) vg[h][k] = ok && FORCE2 ? args.v_grad[3 * oi + k] : 0.0;
           live[h] = !(vr[h] == 0.0 && vg[h][0] == 0.0 && vg[h][1] == 0.0 && vg[h][2] == 0.0);
         }
       }
@@ -562,8 +565,8 @@ __global__ void __launch_bounds__(kFThreads, 1) fp64_tile_kernel(const Fp64Args 
               const int p = h * 32 + lane;
               const double* ap = ao + (int64_t)v * PTS + p;
               const double G0 = sG[v * kFGLd + p];
-              const double Y = MODE == kFForce2 ? sG[v * kFGLd + (PTS % kFRows) + p] : vr[h] * G0;
-              if constexpr (MODE == kFForce2) {
+              const double Y = FORCE2 ? sG[v * kFGLd + (PTS % kFRows) + p] : vr[h] * G0;
+              if constexpr (FORCE2) {
                 double H[6];
 #pragma unroll
                 for (int x = 0; x < 6; ++x) H[x] = __ldg(ap + (4 + x) * ldq);
