@@ -16,7 +16,7 @@
 //    d_i d_j phi, or with d_k phi when the tile has phi rows only.  With rows
 //    phi, d_x, d_y, d_z phi the multiply-adds fall from 4 to about 2.5 per
 //    (mu, nu), with phi rows alone (density only) from 1 to about 1/2.  A D
-//    that is not symmetric (flag of symmetry_kernel) takes the full sums.
+//    that is not symmetric (flag of density_kernel) takes the full sums.
 // 2. Rate.  One persistent CTA per SM with separate warps for the loads, the
 //    matrix instructions and the epilogue, so that index loads, gathers of D
 //    and the epilogue's AO reads run beside the matrix pipe: 4 producer warps

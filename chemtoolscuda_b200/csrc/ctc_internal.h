@@ -20,8 +20,6 @@ int fail(int code, const std::string& msg);
 int ensure_smem_attr(const void* kernel, int bytes);
 // Streaming multiprocessors of the current device (cached per device).
 int device_sm_count(int* out);
-__global__ void permute_density_kernel(const double* __restrict__ D, int M, int Mpad,
-                                       const int32_t* __restrict__ perm, double* __restrict__ out);
 
 #define CTC_CUDA_TRY(expr)                                                               \
   do {                                                                                   \
@@ -148,7 +146,7 @@ struct ctc_molecule {
   int n_aochunk[2] = {0, 0};
   int32_t* d_ao_atom = nullptr;
   double* d_D = nullptr;                     // Mpad x Mpad, zero padded
-  int32_t* d_sym = nullptr;                  // 1: D is symmetric (set_symmetry_flag)
+  int32_t* d_sym = nullptr;                  // not 0: D is symmetric (density_kernel)
   // split-precision copy of D: per row and quad of four columns the plane words
   // of digits 0-3 (16 bytes), then those of digit 4 (4 bytes); row scales
   int8_t* d_Dsl = nullptr;
@@ -227,9 +225,6 @@ int fp64_local_tiles(ctc_molecule* mol, const LocalPlan& plan, const TileBatch& 
 
 // per-point finalisation shared by the contraction kernels (ctc_local.cu)
 struct LocalSums;
-
-// d_sym of the density matrix now in d_D, on the stream.
-int set_symmetry_flag(ctc_molecule* mol, cudaStream_t st);
 
 // Host copy of D (internal order) brought up to date after a device-side
 // replacement (ctc_molecule_set_density_matrix); synchronises the device.
